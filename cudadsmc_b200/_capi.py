@@ -126,6 +126,9 @@ SIGNATURES = [
     ("dsmc_init_from_fields_two_stream", _I, [_P, _P, ctypes.c_float, _P]),
     ("dsmc_gemm_bf16", _I, [_I, _I, _I, _P, _I, _I, _P, _I, _I, _P, _I, ctypes.c_float, _P, _I, _P,
                             _I, _I, _P]),
+    ("dsmc_gemm_split_workspace", ctypes.c_size_t, [_I, _I, _I]),
+    ("dsmc_gemm_split_bf16", _I, [_I, _I, _I, _P, _I, _I, _P, _I, _I, _P, _P, _I, _P, _P]),
+    ("dsmc_decode_mse", _I, [_I, _I, _I, _P, _P, _P, _P, ctypes.c_float, _P, _P, _P, _P, _P, _P]),
     ("dsmc_gemm_check", _I, [_P]),
     ("dsmc_gelu_backward", _I, [_P, _P, _P, _P, ctypes.c_size_t, _P]),
     ("dsmc_colsum", _I, [_P, _I, _I, _I, _P, _P]),

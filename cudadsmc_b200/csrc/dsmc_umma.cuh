@@ -1,76 +1,52 @@
-// BF16 GEMM on the fifth-generation tensor cores (sm_100a): tcgen05.mma with
-// both operands in shared memory, the FP32 accumulator in tensor memory
-// (TMEM), read back by tcgen05.ld for the epilogue.  Used by the warm-start
-// surrogate's layers (dsmc_gemm_bf16); the DSMC timestep has no contraction.
+// Building blocks of the surrogate's BF16 GEMM (dsmc_gemm.cu) on the
+// fifth-generation tensor cores (sm_100a): tcgen05.mma with both operands in
+// shared memory, the FP32 accumulator in tensor memory (TMEM), tiles moved by
+// the tensor memory accelerator (TMA).
 //
-// One CTA of 128 threads computes a 128 x 128 tile of C = A B.  K advances
-// 64 at a time through a two-stage ring of shared-memory tiles: all threads
-// copy the next stage from global memory (16-byte vectors along each
-// operand's contiguous dimension) while the tensor cores work on the
-// current one; one thread issues the four K = 16 MMAs of a stage and commits
-// them to the stage's mbarrier, which frees the stage again.
-//
-// Shared-memory operand layout: the canonical layout without swizzle.  A
-// "core matrix" is 8 rows of 16 bytes (128 bytes, contiguous).  For a K-major
-// operand (K contiguous in global memory) a 16-byte row holds 8 consecutive k
-// of one m (or n); for an MN-major operand it holds 8 consecutive m (or n) of
-// one k.  Core matrices are laid out with the 16 groups of 8 along M (or N)
-// 128 bytes apart (the descriptor's stride byte offset) and the groups of 8
-// along K 2048 bytes apart (its leading byte offset), the same numbers for
-// both majors.
+// Operand tiles use the canonical layouts with the 128-byte swizzle, which
+// is what a TMA box of 128 bytes (64 BF16) by R rows with the same swizzle
+// writes: row r at 128 r bytes, its 16-byte chunk c at position c ^ (r & 7).
+//   K-major operand (K contiguous in memory): one box of 64 k by R rows of M
+//   or N; groups of 8 rows 1024 bytes apart (the descriptor's stride byte
+//   offset); the next 16 k of the tile start 32 bytes on.
+//   MN-major operand (M or N contiguous): per 64 of M or N one box of 64 by
+//   64 k, 8192 bytes apart (the leading byte offset); groups of 8 k 1024
+//   bytes apart (the stride byte offset); the next 16 k start 2048 bytes on.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <cstdint>
 
+#include "dsmc_bulk.cuh"
+
 namespace dsmcb {
 namespace umma {
 
-constexpr int kBM = 128, kBN = 128, kBK = 64, kStages = 2, kThreads = 128;
-constexpr int kTileBytes = kBM * kBK * 2;  // 16 KB per operand tile (kBM == kBN)
-constexpr uint32_t kLbo = 2048;            // between groups of 8 along K
-constexpr uint32_t kSbo = 128;             // between groups of 8 along M / N
-constexpr uint32_t kTmemCols = 128;        // the FP32 accumulator: 128 lanes x 128 columns
-
-struct __align__(128) Smem {
-  __nv_bfloat16 a[kStages][kBM * kBK];
-  __nv_bfloat16 b[kStages][kBN * kBK];
-  unsigned long long mbar[kStages];
-  uint32_t tmem_base;
-  uint32_t failed;
-};
-
-// Byte offset of element (r, k) (r along M or N) in an operand tile.
-__device__ __forceinline__ uint32_t kmajor_off(uint32_t r, uint32_t k) {
-  return (k >> 3) * kLbo + (r >> 3) * kSbo + (r & 7u) * 16u + (k & 7u) * 2u;
-}
-__device__ __forceinline__ uint32_t mnmajor_off(uint32_t r, uint32_t k) {
-  return (k >> 3) * kLbo + (r >> 3) * kSbo + (k & 7u) * 16u + (r & 7u) * 2u;
-}
+constexpr int kBM = 128, kBK = 64;
 
 // Shared-memory matrix descriptor: start address, leading and stride byte
-// offsets (all in 16-byte units), version 1 (sm100), no swizzle.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
+// offsets (all in 16-byte units), version 1 (sm100), 128-byte swizzle.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((kLbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((kSbo >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)(1024u >> 4) << 32;
   d |= (uint64_t)1u << 46;
+  d |= (uint64_t)2u << 61;
   return d;
 }
 
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B,
-// operand majors (0 K, 1 MN), N = 128, M = 128.
-__host__ __device__ constexpr uint32_t instr_desc(uint32_t a_mn, uint32_t b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn << 15) | (b_mn << 16) |
-         ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+// operand majors (0 K, 1 MN), M = 128.
+__host__ __device__ constexpr uint32_t instr_desc(uint32_t a_mn, uint32_t b_mn, uint32_t n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn << 15) | (b_mn << 16) | ((n >> 3) << 17) |
+         ((uint32_t)(kBM >> 4) << 24);
 }
 
-__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(dst_smem)),
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dev::smem_u32(dst_smem)),
                "r"(ncols)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -93,7 +69,7 @@ __device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t a, uint64_t b, uin
 }
 __device__ __forceinline__ void commit(unsigned long long* mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   su32(mbar))
+                   dev::smem_u32(mbar))
                : "memory");
 }
 // 32 consecutive FP32 columns of this thread's TMEM lane.
@@ -113,6 +89,41 @@ __device__ __forceinline__ void ld32(uint32_t taddr, float (&v)[32]) {
 #pragma unroll
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
+
+__device__ __forceinline__ void mbar_arrive(unsigned long long* m) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dev::smem_u32(m)) : "memory");
+}
+
+// TMA, two-dimensional tiles (x: the contiguous dimension).
+__device__ __forceinline__ void tma_prefetch(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int x, int y,
+                                         unsigned long long* mbar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+          dev::smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(dev::smem_u32(mbar))
+      : "memory");
+}
+__device__ __forceinline__ void tma_store(const CUtensorMap* map, const void* src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x),
+               "r"(y), "r"(dev::smem_u32(src))
+               : "memory");
+}
+__device__ __forceinline__ void tma_reduce_add(const CUtensorMap* map, const void* src, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map),
+               "r"(x), "r"(y), "r"(dev::smem_u32(src))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// at most the N newest of this thread's store groups still reading shared
+// memory
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 }  // namespace umma
 }  // namespace dsmcb

@@ -85,9 +85,8 @@ class WarmStartMLP:
         return out
 
     # ------------------------------------------------------------ forward --
-    def forward(self, x):
-        """x: [batch, n_in] normalized inputs.  Returns the field [batch, F]
-        (FP32, on the device) and the cache for backward."""
+    def _coefficients(self, x):
+        """The hidden layers and the coefficients: the cache for backward."""
         torch = self.torch
         B = len(x)
         h = self._inputs(x)
@@ -107,8 +106,15 @@ class WarmStartMLP:
         self._gemm(B, self.modes, self.hidden, h, self.hidden, 0, self.bf["Wout"], self.modes, 0, c,
                    self.modes, bias=self.params["bout"], cb=cb, ldcb=self.modes)
         cache["c"] = cb
-        y = torch.empty((B, self.F), dtype=torch.float32, device=self.dev)
-        self._gemm(B, self.F, self.modes, cb, self.modes, 0, self.bf["B"], self.F, 0, y, self.F,
+        return cache
+
+    def forward(self, x):
+        """x: [batch, n_in] normalized inputs.  Returns the field [batch, F]
+        (FP32, on the device) and the cache for backward."""
+        B = len(x)
+        cache = self._coefficients(x)
+        y = self.torch.empty((B, self.F), dtype=self.torch.float32, device=self.dev)
+        self._gemm(B, self.F, self.modes, cache["c"], self.modes, 0, self.bf["B"], self.F, 0, y, self.F,
                    bias=self.params["mean"])
         return y, cache
 
@@ -118,25 +124,26 @@ class WarmStartMLP:
         Returns (loss, valid count, grads dict of FP32 tensors)."""
         torch = self.torch
         B = len(x)
-        y, cache = self.forward(x)
+        cache = self._coefficients(x)
+        y = torch.empty((B, self.F), dtype=torch.float32, device=self.dev)
         n = B * self.F
-        dy = torch.empty_like(y)
         dyb = torch.empty(y.shape, dtype=torch.bfloat16, device=self.dev)
         acc = torch.zeros(1, dtype=torch.float64, device=self.dev)
         cnt = torch.zeros(1, dtype=torch.int64, device=self.dev)
-        check(lib().dsmc_mse_grad(_p(y), _p(targets_bf16), n, 1.0 / n, _p(dyb), _p(dy), _p(acc), _p(cnt),
-                                  _stream()), "mse_grad")
         g = {}
+        g["mean"] = torch.empty(self.F, dtype=torch.float32, device=self.dev)
+        check(lib().dsmc_decode_mse(B, self.F, self.modes, _p(cache["c"]), _p(self.bf["B"]),
+                                    _p(self.params["mean"]), _p(targets_bf16), 1.0 / n, _p(y), _p(dyb),
+                                    _p(g["mean"]), _p(acc), _p(cnt), _stream()), "decode_mse")
         g["B"] = torch.empty((self.modes, self.F), dtype=torch.float32, device=self.dev)
         self._gemm(self.modes, self.F, B, cache["c"], self.modes, 1, dyb, self.F, 0, g["B"], self.F)
-        g["mean"] = torch.empty(self.F, dtype=torch.float32, device=self.dev)
-        check(lib().dsmc_colsum(_p(dy), B, self.F, self.F, _p(g["mean"]), _stream()), "colsum")
-        dc = torch.zeros((B, self.modes), dtype=torch.float32, device=self.dev)
-        split = max(1, min(64, self.F // 4096))
-        self._gemm(B, self.modes, self.F, dyb, self.F, 0, self.bf["B"], self.F, 1, dc, self.modes,
-                   split=split)
+        dc = torch.empty((B, self.modes), dtype=torch.float32, device=self.dev)
         dcb = torch.empty(dc.shape, dtype=torch.bfloat16, device=self.dev)
-        check(lib().dsmc_to_bf16(_p(dc), _p(dcb), dc.numel(), _stream()), "to_bf16")
+        split = max(1, min(64, self.F // 4096))
+        ws = torch.empty(lib().dsmc_gemm_split_workspace(B, self.modes, split), dtype=torch.uint8,
+                         device=self.dev)
+        check(lib().dsmc_gemm_split_bf16(B, self.modes, self.F, _p(dyb), self.F, 0, _p(self.bf["B"]), self.F, 1,
+                                         _p(dc), _p(dcb), split, _p(ws), _stream()), "gemm_split_bf16")
         g["Wout"] = torch.empty((self.hidden, self.modes), dtype=torch.float32, device=self.dev)
         self._gemm(self.hidden, self.modes, B, cache["h"], self.hidden, 1, dcb, self.modes, 0, g["Wout"],
                    self.modes)

@@ -535,6 +535,21 @@ int dsmc_stage_sample(const float* u, const float* v, const float* w, const uint
 int dsmc_gemm_bf16(int m, int n, int k, const void* a, int lda, int a_trans, const void* b, int ldb,
                    int b_trans, float* c, int ldc, float beta, const float* bias, int act, void* c_bf16,
                    int ldcb, int split_k, void* stream);
+/* c = A B with the reduction in split_k parts, each part's FP32 product kept
+ * in the workspace (dsmc_gemm_split_workspace bytes, 16-byte aligned) and the
+ * parts added in FP64: the same result on every call.  c (and c_bf16, when
+ * given) m x n without padding; n a multiple of 4; the other conditions of
+ * dsmc_gemm_bf16. */
+size_t dsmc_gemm_split_workspace(int m, int n, int split_k);
+int dsmc_gemm_split_bf16(int m, int n, int k, const void* a, int lda, int a_trans, const void* b, int ldb,
+                         int b_trans, float* c, void* c_bf16, int split_k, float* workspace, void* stream);
+/* The decoder and its error in one pass: y = A B + bias (A m x k, B k x n,
+ * all arrays row-major without padding), and with the masked mean-square
+ * error of dsmc_mse_grad against t: loss, count, dy in BF16 and the column
+ * sums of dy in FP32.  k and n multiples of 8, A and B 16-byte aligned. */
+int dsmc_decode_mse(int m, int n, int k, const void* a, const void* b, const float* bias, const void* t_bf16,
+                    float scale, float* y, void* dy_bf16, float* dy_colsum, double* loss,
+                    unsigned long long* count, void* stream);
 /* Synchronises `stream` and reports whether a dsmc_gemm_bf16 launch since
  * the last check gave up waiting on its tensor-core work (DSMC_ERR_DEVICE;
  * its output is then incomplete); clears the flag. */
