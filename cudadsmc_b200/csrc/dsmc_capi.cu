@@ -133,14 +133,25 @@ void drop_graph(dsmc_handle* h) {
 }
 
 // Cell-kernel variant and the tile size that goes with it: tiles of about one
-// shared-memory chunk of particles (32..256 cells); the warp-autonomous
-// variants use tiles of 32 cells, one per lane.
+// shared-memory chunk of particles (32..256 cells).  The warp-autonomous
+// variants give each warp a tile of at most 32 cells, one per lane: 32 where
+// that makes enough tiles for the warps of one wave, fewer on small grids,
+// where a warp's chain of chunks is the kernel's length (order kernel, 16^3
+// cells of 24: 36 us with 32, 13 with 4; 13,824 cells of 8: 16 with 32, 10
+// with 8; 65,536 cells: 18 with 32, 20 with 16), and 16 where they fill a
+// chunk and there are tiles enough to even out (524,288 cells of 6-8: 89 with
+// 32, 84 with 16; 182,250 cells of 9: 37 with 32, 40 with 16).
 void apply_variant(dsmc_handle* h, int v) {
   h->variant = v;
   const uint64_t cap = (uint64_t)dsmcb::cell_kernel_chunk_capacity(v);
   uint32_t ct = dsmcb::kMaxCellsPerTile;
   while (ct > 32 && (uint64_t)ct * std::max<uint32_t>(h->ppc, 1) > cap) ct >>= 1;
-  if (dsmcb::cell_kernel_is_warp(v)) ct = dsmcb::cell_kernel_w_tile();
+  if (dsmcb::cell_kernel_is_warp(v)) {
+    const uint64_t wave = (uint64_t)dsmcb::num_sms() * 20u;  // resident warps of the default shape
+    ct = dsmcb::cell_kernel_w_tile();
+    while (ct > 4 && 2u * ((uint64_t)h->cells / ct) < wave) ct >>= 1;
+    if (ct == 32 && (uint64_t)h->cells >= 16u * 8u * wave && 16u * (uint64_t)h->ppc * 10u >= 9u * cap) ct = 16;
+  }
   h->cells_per_tile = ct;
   h->n_tiles = (h->cells + ct - 1) / ct;
   drop_graph(h);
@@ -2041,12 +2052,14 @@ int batch_capture(dsmc_batch* b, const std::vector<float>& dt) {
     np[i] = (double)m.n_alive + (double)m.n_pending + 1.0;
     nc[i] = (double)h->cells;
     // every member runs the split kernels with the order kernel's
-    // (128 particles, 4 warps, 5 CTAs) shape and tiles of 32 cells, whatever
-    // shape it uses stepped alone
+    // (128 particles, 4 warps, 5 CTAs) shape and tiles of 32 cells (16 in
+    // dense members, whose 16 cells make more than one chunk: 919 -> 912 us
+    // per step of 32 members), whatever shape it uses stepped alone
     P[i] = step_params(h, dt[i], true);
     P[i].cell_variant = 5;
-    P[i].cells_per_tile = (int)dsmcb::cell_kernel_w_tile();
-    P[i].n_tiles = (h->cells + dsmcb::cell_kernel_w_tile() - 1) / dsmcb::cell_kernel_w_tile();
+    const uint32_t ct = dsmcb::cell_kernel_w_tile() >> (h->ppc >= 12 ? 1 : 0);
+    P[i].cells_per_tile = (int)ct;
+    P[i].n_tiles = (h->cells + ct - 1) / ct;
     A[i] = dsmcb::SortArgs{h->count, h->cursor, h->start, h->tile_sum, h->orig, h->keys,
                            h->meta, h->cells, h->n_scan_tiles, h->capacity};
     for (const auto& in : h->inflows) I.push_back(inject_params(h, in, dt[i], P[i].seed));

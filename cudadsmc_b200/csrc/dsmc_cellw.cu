@@ -1,8 +1,8 @@
 // The timestep's cell work as warp-autonomous kernels (sm_100a); none has a
 // CTA-wide barrier inside its loop.
 //
-// k_order_w (order + pair counts): warps take tiles of 32 consecutive cells
-// (lane L owns cell L; tiles past the first wave come from a dynamic counter)
+// k_order_w (order + pair counts): warps take tiles of up to 32 consecutive
+// cells (lane L owns cell L; a warp's third tile and on come from a dynamic counter)
 // and cut them into chunks of whole cells holding at most CAPW particles.  A
 // chunk's orig (the pre-scatter index of every sorted slot) is staged in the
 // warp's slice of shared memory by a 1-D bulk copy completing on the warp's
@@ -40,7 +40,7 @@ namespace {
 
 using namespace dev;
 
-constexpr uint32_t kWarpTile = 32;  // cells per warp tile, one per lane
+constexpr uint32_t kWarpTile = 32;  // most cells per warp tile, one per lane (StepParams::cells_per_tile)
 constexpr uint32_t kFlightQ = 64;   // per-warp queue of flights that may reach the body
 
 template <int CAPW>
@@ -57,8 +57,9 @@ constexpr size_t collide_smem_bytes() {
   return WARPS * sizeof(WarpSmem<CAPW>);
 }
 
-// A tile of 32 cells as the lanes see it: lane L holds the start and end of
-// cell 32 t + L (cells past the last one are empty at the total count).
+// A tile of C = cells_per_tile cells as the lanes see it: lane L < C holds the
+// start and end of cell C t + L (cells past the last one are empty at the
+// total count).
 struct WTile {
   uint32_t t, nct, s, e;
 };
@@ -69,23 +70,25 @@ __device__ __forceinline__ WTile load_tile(const StepParams& p, uint32_t t) {
   w.nct = 0;
   w.s = w.e = 0;
   if (t < p.n_tiles) {
-    const uint32_t c0 = t * kWarpTile;
+    const uint32_t c0 = t * (uint32_t)p.cells_per_tile;
     const uint32_t c = c0 + lane_id();
-    w.nct = min(kWarpTile, p.cells - c0);
+    w.nct = min((uint32_t)p.cells_per_tile, p.cells - c0);
     w.s = __ldg(&p.start[min(c, p.cells)]);
     w.e = __ldg(&p.start[min(c + 1u, p.cells)]);
   }
   return w;
 }
 
-// Tiles of a warp: tile w first, then from the step's dynamic counter (or
-// round robin without one).  Lane 0 asks ahead of need so that the atomic's
-// latency is hidden.
+// Tiles of a warp: tiles w and w + (number of warps) first, then from the
+// step's dynamic counter (or round robin without one).  Lane 0 asks ahead of
+// need so that the atomic's latency is hidden.  (With the second tile asked
+// for as well, a grid of two tiles per warp gave half the warps three and the
+// others one.)
 struct TileQueue {
   uint32_t nwarps, next_static;
   uint32_t* counter;
   __device__ __forceinline__ uint32_t grab() {
-    if (counter) return nwarps + atomicAdd(counter, 1u);
+    if (counter) return 2u * nwarps + atomicAdd(counter, 1u);
     const uint32_t t = next_static;
     next_static += nwarps;
     return t;
@@ -214,9 +217,9 @@ __device__ __forceinline__ uint32_t stable_slot(const uint32_t* ORA, const uint3
   return pos;
 }
 
-// Appends e for every lane with `put` to list (one atomic per warp; all lanes
-// call it).
-__device__ __forceinline__ void list_cells(uint4* list, uint32_t* counter, bool put, uint4 e) {
+// Appends e for every lane with `put` to list, which grows by `dir` (one
+// atomic per warp; all lanes call it).
+__device__ __forceinline__ void list_cells(uint4* list, int dir, uint32_t* counter, bool put, uint4 e) {
   const uint32_t lane = lane_id();
   const unsigned m = __ballot_sync(kFull, put);
   if (!m) return;
@@ -224,7 +227,7 @@ __device__ __forceinline__ void list_cells(uint4* list, uint32_t* counter, bool 
   uint32_t base = 0;
   if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
   base = __shfl_sync(kFull, base, leader);
-  if (put) list[base + __popc(m & ((1u << lane) - 1u))] = e;
+  if (put) list[dir * (int)(base + __popc(m & ((1u << lane) - 1u)))] = e;
 }
 
 // Adds v, summed over the block, to *dst with one atomic (every thread of the
@@ -301,14 +304,11 @@ __device__ __forceinline__ void order_body(const StepParams& p, const uint32_t v
 
   const uint32_t nwarps = vg * WARPS;
   const uint32_t gw = vb * WARPS + warp;
-  TileQueue tq{nwarps, gw + nwarps, p.meta ? &p.meta->tile_next : nullptr};
+  TileQueue tq{nwarps, gw + 2u * nwarps, p.meta ? &p.meta->tile_next : nullptr};
   WTile A = load_tile(p, gw);
-  uint32_t pend = 0, tb = 0;
-  if (lane == 0 && gw < p.n_tiles) {
-    tb = tq.grab();
-    pend = tq.grab();
-  }
-  tb = __shfl_sync(kFull, gw < p.n_tiles ? tb : 0xffffffffu, 0);
+  const uint32_t tb = gw + nwarps;
+  uint32_t pend = 0;
+  if (lane == 0 && tb < p.n_tiles) pend = tq.grab();
   WTile B = load_tile(p, tb);
 
   uint32_t phase = 0;  // bit b: parity of the next phase of buffer b
@@ -351,7 +351,7 @@ __device__ __forceinline__ void order_body(const StepParams& p, const uint32_t v
   float2 mr_c = make_float2(0.f, 0.f);
   auto load_cell_state = [&](const WChunk& K, uint32_t tile, float2& mr) {
     if (do_collide && K.valid && !K.giant && K.n && lane >= K.cur && lane < K.cur + K.k)
-      mr = p.maxrem[tile * kWarpTile + lane];
+      mr = p.maxrem[tile * (uint32_t)p.cells_per_tile + lane];
   };
   if (A.t < p.n_tiles) {
     C = make_wchunk<CAPW>(A, 0, 0);
@@ -375,7 +375,7 @@ __device__ __forceinline__ void order_body(const StepParams& p, const uint32_t v
     float2 mr_n = make_float2(0.f, 0.f);
     load_cell_state(N, n_in_b ? B.t : A.t, mr_n);
 
-    const uint32_t c0 = A.t * kWarpTile;
+    const uint32_t c0 = A.t * (uint32_t)p.cells_per_tile;
     const uint32_t cell = c0 + lane;
     const bool mine = lane >= C.cur && lane < C.cur + C.k;
     const uint32_t s0 = A.s - C.base, nc = A.e - A.s;  // meaningful for `mine`
@@ -471,7 +471,9 @@ __device__ __forceinline__ void order_body(const StepParams& p, const uint32_t v
         const bool heavy = heavy_mode && M >= kHeavyMin;
         const uint4 e = make_uint4(cell, base + s0, nc, M);
         buffer_cells(S.lbuf, lcnt, p.ntc_light, &p.meta->n_light, M > 0 && !heavy, e);
-        list_cells(p.ntc_heavy, &p.meta->n_heavy, heavy, e);
+        const bool heaviest = heavy && M >= kHeaviestMin;
+        list_cells(p.ntc_heavy, 1, &p.meta->n_heaviest, heaviest, e);
+        list_cells(p.ntc_heavy + (p.cells - 1u), -1, &p.meta->n_heavy, heavy && !heaviest, e);
       }
       cp_async_commit();
       // C: the previous chunk, in sorted order, to the mid arrays while this
@@ -518,13 +520,20 @@ constexpr uint32_t kNtcClaim = 256;  // claim slots per warp: the largest chunk
 // The pair counts and remainders come from k_order_w; this kernel updates
 // (sigma g)max (and the HybridTaus state in the reference RNG mode) with the
 // same arithmetic and random streams as the fused path.  The grid is one
-// wave: dense cells (the longest chains) go first, a warp each, then warps
-// claim light cells 32 at a time, so that the warps that finish early take
-// more (with a static split the blocks holding both a second round of light
-// cells and a dense cell set the kernel's length).
+// wave.  What bounds it is each warp's chain (6 us per item on a 4M-particle
+// flow: entry, velocities, then one pair or round after the other), so the
+// dense cells go first, the longest of them (kHeaviestMin) before the others,
+// and the rest is claimed as warps come free; with fewer light cells than
+// lanes nothing is claimed, and every warp takes one share (16^3 cells:
+// 20 -> 14 us; 65,536 cells: 24 -> 18 us; the claims of 3,500 warps on one
+// counter were the difference).  A dense cell's velocities sit in shared
+// memory and its random words come a block at a time (64x32x32 sphere flow,
+// 27 -> 19 us with the claims).  The two-CTA register cap keeps it free of
+// spills: 3 CTAs ran the sphere flow's 3 us slower, the capsule's 1 us faster.
 template <int WARPS>
 __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb, const uint32_t vg) {
   __shared__ uint32_t s_claim[WARPS][kNtcClaim];
+  __shared__ float s_vel[WARPS][3][kNtcClaim];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t step = p.step_override ? p.step_override : p.meta->step;
   const bool taus = p.rng_kind == 0;
@@ -532,39 +541,68 @@ __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb,
   __syncwarp();
   uint32_t col = 0;
   double sum_g = 0.0;
-  const uint32_t nl = p.meta->n_light, nh = p.meta->n_heavy;
+  const uint32_t nl = p.meta->n_light, nh1 = p.meta->n_heaviest, nh = nh1 + p.meta->n_heavy;
   const uint32_t gw = vb * WARPS + warp, nw = vg * WARPS;
-  for (uint32_t h = gw; h < nh; h += nw) {
-    const uint4 e = p.ntc_heavy[h];
-    GlobalVel acc{p.mid.u, p.mid.v, p.mid.w, e.y};
-    const float2 vm = p.maxrem[e.x];  // .y: the remainder k_order_w stored
-    const float vmax =
-        ntc_select_heavy_warp(p, e.x, e.z, acc, s_claim[warp], step, e.w, vm.x, col, sum_g);
-    __syncwarp();
-    if (lane == 0) p.maxrem[e.x] = make_float2(vmax, vm.y);
-  }
+  const uint32_t nlw = nw > nh ? nw - nh : 0u;  // warps without a dense cell
+  // few cells: one item per warp and no claims, the light cells spread over
+  // all warps that have no dense one
+  const bool once = nlw > 0u && nl <= 32u * nlw;
+  const uint32_t per = once ? (nl + nlw - 1u) / nlw : 32u;
+  // items: the dense cells, the longest chains first, then the light cells
+  // `per` at a time; item gw first, then from the step's counter, the next
+  // one asked for ahead of need (but not behind the longest chains, where it
+  // would wait for their end)
+  const uint32_t items = nh + (per ? (nl + per - 1u) / per : 0u);
   uint32_t* claims = &p.meta->tile_next2;
-  uint32_t next = 0;
-  if (lane == 0) next = atomicAdd(claims, 32u);
-  for (uint32_t base = __shfl_sync(kFull, next, 0); base < nl;) {
-    // the claim after this one, asked for ahead of need
-    if (lane == 0) next = atomicAdd(claims, 32u);
-    const uint32_t i = base + lane;
-    base = __shfl_sync(kFull, next, 0);
-    if (i >= nl) continue;
-    const uint4 e = p.ntc_light[i];  // cell, first sorted slot, count, pairs
-    GlobalVel acc{p.mid.u, p.mid.v, p.mid.w, e.y};
-    float2 vm = p.maxrem[e.x];
-    if (taus) {
-      TausRng r;
-      r.s = p.seeds[e.x];
-      float4 stat = make_float4(0.f, 0.f, 0.f, 0.f);
-      ntc_select_reference(p, (int)e.z, acc, r, e.w, vm, stat, col, sum_g);
-      p.seeds[e.x] = r.s;
+  for (uint32_t it = once ? (gw < nlw ? nh + gw : gw - nlw) : gw; it < items;) {
+    const bool ahead = it >= nh1;
+    uint32_t next = items;
+    if (!once && ahead && lane == 0) next = nw + atomicAdd(claims, 1u);
+    if (it < nh) {
+      const uint4 e = p.ntc_heavy[it < nh1 ? it : p.cells - 1u - (it - nh1)];
+      // the cell's velocities in shared memory for the selections: its rounds
+      // are one warp's chain, and every particle is touched several times
+      float* su = s_vel[warp][0];
+      float* sv = s_vel[warp][1];
+      float* sw = s_vel[warp][2];
+      for (uint32_t t = lane; t < e.z; t += 32) {
+        su[t] = p.mid.u[e.y + t];
+        sv[t] = p.mid.v[e.y + t];
+        sw[t] = p.mid.w[e.y + t];
+      }
+      const float2 vm = p.maxrem[e.x];  // .y: the remainder k_order_w stored
+      __syncwarp();
+      GlobalVel acc{su, sv, sw, 0u};
+      const float vmax =
+          ntc_select_heavy_warp(p, e.x, e.z, acc, s_claim[warp], step, e.w, vm.x, col, sum_g);
+      __syncwarp();
+      for (uint32_t t = lane; t < e.z; t += 32) {
+        p.mid.u[e.y + t] = su[t];
+        p.mid.v[e.y + t] = sv[t];
+        p.mid.w[e.y + t] = sw[t];
+      }
+      if (lane == 0) p.maxrem[e.x] = make_float2(vmax, vm.y);
     } else {
-      col += ntc_select_fast(p, e.x, e.z, acc, step, e.w, vm, sum_g);
+      const uint32_t i = (it - nh) * per + lane;
+      if (lane < per && i < nl) {
+        const uint4 e = p.ntc_light[i];  // cell, first sorted slot, count, pairs
+        GlobalVel acc{p.mid.u, p.mid.v, p.mid.w, e.y};
+        float2 vm = p.maxrem[e.x];
+        if (taus) {
+          TausRng r;
+          r.s = p.seeds[e.x];
+          float4 stat = make_float4(0.f, 0.f, 0.f, 0.f);
+          ntc_select_reference(p, (int)e.z, acc, r, e.w, vm, stat, col, sum_g);
+          p.seeds[e.x] = r.s;
+        } else {
+          col += ntc_select_fast(p, e.x, e.z, acc, step, e.w, vm, sum_g);
+        }
+        p.maxrem[e.x] = vm;
+      }
     }
-    p.maxrem[e.x] = vm;
+    if (!once && !ahead && lane == 0) next = nw + atomicAdd(claims, 1u);
+    __syncwarp();
+    it = __shfl_sync(kFull, next, 0);
   }
   __shared__ unsigned long long s_col[WARPS];
   __shared__ double s_g[WARPS];
@@ -575,12 +613,12 @@ __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb,
 }
 
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) k_ntc_w(const __grid_constant__ StepParams p) {
+__global__ void __launch_bounds__(WARPS * 32, 2) k_ntc_w(const __grid_constant__ StepParams p) {
   chained_entry();
   ntc_body<WARPS>(p, blockIdx.x, gridDim.x);
 }
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) k_ntc_wb(const __grid_constant__ BatchOf<StepParams> bv) {
+__global__ void __launch_bounds__(WARPS * 32, 5) k_ntc_wb(const __grid_constant__ BatchOf<StepParams> bv) {
   chained_entry();
   uint32_t vb, vg;
   const StepParams& p = bv.locate(vb, vg);
@@ -1205,6 +1243,7 @@ cudaError_t launch_flight_pw(const StepParams& p, cudaStream_t stream) {
 }
 
 constexpr int kNtcWarps = 8;
+constexpr int kNtcWarpsB = 4;  // batched: 20 warps per SM without spills
 
 cudaError_t launch_ntc_w(const StepParams& p, cudaStream_t stream) {
   static LaunchShapeW cache[8];
@@ -1300,7 +1339,7 @@ cudaError_t cell_batch_waves(uint32_t wave[5], size_t flight_smem) {
   if (e != cudaSuccess) return e;
   int per[5] = {0, 0, 0, 0, 0};
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0], k_order_wb<128, 4, 5>, 128, osmem);
-  if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_ntc_wb<kNtcWarps>, kNtcWarps * 32, 0);
+  if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_ntc_wb<kNtcWarpsB>, kNtcWarpsB * 32, 0);
   if (!e)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_flight_wb<kFlightWarps, 4>, kFlightWarps * 32,
                                                       flight_smem);
@@ -1319,7 +1358,7 @@ cudaError_t launch_cell_stage_b(int stage, const BatchOf<StepParams>& bv, uint32
   if (blocks == 0) return cudaSuccess;
   switch (stage) {
     case 0: return launch_chained(k_order_wb<128, 4, 5>, blocks, 128, collide_smem_bytes<128, 4>(), stream, false, bv);
-    case 1: return launch_chained(k_ntc_wb<kNtcWarps>, blocks, kNtcWarps * 32, 0, stream, false, bv);
+    case 1: return launch_chained(k_ntc_wb<kNtcWarpsB>, blocks, kNtcWarpsB * 32, 0, stream, false, bv);
     case 2: return launch_chained(k_flight_wb<kFlightWarps, 4>, blocks, kFlightWarps * 32, flight_smem, stream, false, bv);
     case 3:
       return coop_mesh ? launch_chained(k_mesh_wb<2, true>, blocks, 32 * kMeshWarps, 0, stream, false, bv)

@@ -66,12 +66,8 @@ static __device__ __noinline__ uint4 philox_block(uint32_t b, uint32_t c1, uint3
 }
 
 // A Philox stream: (key, counter words 1..3 fixed) and a running block index
-// in word 0; hands out 32-bit words four at a time.  INLINE_REFILL expands
-// the ten rounds at the draw site (the collision loops, where a call per
-// refill costs more than the code size); elsewhere the refill is the
-// out-of-line philox_block.  Both give the same words.
-template <bool INLINE_REFILL>
-struct PhiloxStreamT {
+// in word 0; hands out 32-bit words four at a time.
+struct PhiloxStream {
   uint2 key;
   uint32_t c1, c2, c3;
   uint32_t block;
@@ -82,8 +78,7 @@ struct PhiloxStreamT {
   }
   __device__ __forceinline__ uint32_t next() {
     if (used == 4) {
-      buf = INLINE_REFILL ? philox4x32_10(make_uint4(block, c1, c2, c3), key)
-                          : philox_block(block, c1, c2, c3, key);
+      buf = philox_block(block, c1, c2, c3, key);
       block++;
       used = 0;
     }
@@ -96,8 +91,48 @@ struct PhiloxStreamT {
     return ((float)(next() >> 8) + 0.5f) * (1.0f / 16777216.0f);
   }
 };
-using PhiloxStream = PhiloxStreamT<false>;
-using PhiloxStreamInline = PhiloxStreamT<true>;
+
+// The same stream for the collision loops: up to eight words held, and
+// ready<N>() makes at least N (at most 5) available, so that a pair's draws
+// have one place where a block is computed.  With a check at every draw the
+// lanes of a warp, each at its own position of its stream, ran the ten rounds
+// up to five times per pair, one after the other.
+struct PhiloxAhead {
+  uint2 key;
+  uint32_t c1, c2, c3;
+  uint32_t block;
+  uint4 a, b;  // words 0-3 and 4-7
+  uint32_t pos, have;
+  __device__ __forceinline__ void init(uint2 k, uint32_t x, uint32_t y, uint32_t z) {
+    key = k; c1 = x; c2 = y; c3 = z; block = 0; pos = 0; have = 0;
+    a = b = make_uint4(0u, 0u, 0u, 0u);
+  }
+  template <uint32_t N>
+  __device__ __forceinline__ void ready() {
+    while (have - pos < N) {
+      while (pos >= 4u) {
+        a = b;
+        pos -= 4u;
+        have -= 4u;
+      }
+      const uint4 w = philox4x32_10(make_uint4(block, c1, c2, c3), key);
+      block++;
+      if (have == 0u) a = w;
+      else b = w;
+      have += 4u;
+    }
+  }
+  __device__ __forceinline__ uint32_t next() {
+    const bool hi = pos >= 4u;
+    const uint32_t x = hi ? b.x : a.x, y = hi ? b.y : a.y, z = hi ? b.z : a.z, w = hi ? b.w : a.w;
+    const uint32_t r = (pos & 2u) ? ((pos & 1u) ? w : z) : ((pos & 1u) ? y : x);
+    pos++;
+    return r;
+  }
+  __device__ __forceinline__ float uniform() {
+    return ((float)(next() >> 8) + 0.5f) * (1.0f / 16777216.0f);
+  }
+};
 
 // ------------------------------------------------------------ geometry ----
 

@@ -150,6 +150,7 @@ __device__ __forceinline__ void scan_body(uint32_t* count, uint32_t* cursor, uin
     meta->n_defer = 0;
     meta->n_light = 0;
     meta->n_heavy = 0;
+    meta->n_heaviest = 0;
     if (bump) {
       meta->step += 1;
       meta->particle_steps += run;

@@ -66,7 +66,9 @@ struct Meta {
   uint32_t tile_next2;   // the NTC kernel's claims of light cells (reset by the scan)
   uint32_t n_defer;      // flights listed for the mesh kernel this step (reset by the scan)
   uint32_t n_light;      // cells listed for the NTC kernel, one lane each (reset by the scan)
-  uint32_t n_heavy;      // cells listed for the NTC kernel, one warp each (reset by the scan)
+  uint32_t n_heavy;      // cells listed for the NTC kernel, one warp each (reset by the scan),
+  uint32_t n_heaviest;   // and those of them with the longest chains, listed apart (in what was
+                         // padding: the struct is part of the snapshot format)
   unsigned long long particle_steps;  // sum over steps of the particles placed by the scan
 };
 
@@ -213,8 +215,8 @@ cudaError_t launch_cell(const StepParams& p, cudaStream_t stream);
 // 4 (256, 4, 4), 5 (128, 4, 5), 6 (128, 8, 3), 7 (128, 4, 6).
 int cell_kernel_variants();
 int cell_kernel_chunk_capacity(int variant);
-// Variants at or above 4 use the warp-autonomous kernel, whose tiles are
-// cell_kernel_w_tile() cells (one per lane).
+// Variants at or above 4 use the warp-autonomous kernel, whose tiles are at
+// most cell_kernel_w_tile() cells (one per lane).
 bool cell_kernel_is_warp(int variant);
 int cell_kernel_w_variants();
 int cell_kernel_w_capacity(int v);

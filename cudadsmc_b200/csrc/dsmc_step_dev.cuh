@@ -10,6 +10,8 @@ namespace dev {
 constexpr unsigned kFull = 0xffffffffu;
 // NTC selections at which a cell is collided by a whole warp (Philox mode).
 constexpr uint32_t kHeavyMin = 8;
+// Selections from which a cell is listed apart, to be started first.
+constexpr uint32_t kHeaviestMin = 32;
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
@@ -265,15 +267,19 @@ template <class Acc>
 __device__ __forceinline__ uint32_t ntc_select_fast(const StepParams& p, uint32_t cell, uint32_t n,
                                                     Acc acc, uint32_t step, uint32_t M, float2& vm,
                                                     double& sum_g) {
-  PhiloxStreamInline r, q;
-  r.init(p.seed, cell, step, kPurposeCollide);
-  q.init(p.seed, cell, step, kPurposePairs);
   uint32_t ncol = 0;
   if (M == 0) return 0;
+  PhiloxAhead r;
+  r.init(p.seed, cell, step, kPurposeCollide);
+  // the pair stream: two words a pair, a block every other pair
+  uint4 qb = make_uint4(0u, 0u, 0u, 0u);
+  uint32_t drawn = 0;
   auto draw = [&](uint32_t& a, uint32_t& b) {
-    a = __umulhi(q.next(), n);
-    b = a + 1u + __umulhi(q.next(), n - 1u);
+    if (!(drawn & 1u)) qb = philox4x32_10(make_uint4(drawn >> 1, cell, step, kPurposePairs), p.seed);
+    a = __umulhi((drawn & 1u) ? qb.z : qb.x, n);
+    b = a + 1u + __umulhi((drawn & 1u) ? qb.w : qb.y, n - 1u);
     if (b >= n) b -= n;
+    drawn++;
   };
   uint32_t pi, pj;
   draw(pi, pj);
@@ -289,6 +295,7 @@ __device__ __forceinline__ uint32_t ntc_select_fast(const StepParams& p, uint32_
     }
     const float mag = rel_speed(v1, v2);
     const float v = sigma_g_fast(p, mag);
+    r.ready<3>();
     if (v > r.uniform() * vm.x) {
       ncol++;
       sum_g += mag;
@@ -356,7 +363,7 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
                                                        uint32_t& col, double& sum_g) {
   const unsigned lane = lane_id();
   float vmax = vmax_in;
-  PhiloxStreamInline rng;
+  PhiloxAhead rng;
   rng.init(p.seed, cell, step, kPurposeHeavy + lane);
   uint32_t drawn = 0, done = 0, pi = 0, pj = 0, ncol = 0;
   bool pend = false;
@@ -364,6 +371,7 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
     const unsigned idle = __ballot_sync(kFull, !pend);
     const uint32_t want = min((uint32_t)__popc(idle), M - drawn);
     const uint32_t r = __popc(idle & ((1u << lane) - 1u));
+    rng.ready<5>();  // a round's draws: two for the pair, one to accept, two to scatter
     if (!pend && r < want) {
       pi = __umulhi(rng.next(), n);
       pj = pi + 1u + __umulhi(rng.next(), n - 1u);
@@ -402,10 +410,8 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
     }
     if (win) pend = false;
     done += __popc(__ballot_sync(kFull, win));
-    float mx = vv;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
-    vmax = fmaxf(vmax, mx);
+    // (not negative: the order of the bits is the order of the values)
+    vmax = fmaxf(vmax, __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(vv))));
     __syncwarp();
   }
   col += ncol;
