@@ -373,7 +373,7 @@ dsmcb::StepParams step_params(dsmc_handle* h, float dt, bool split) {
   p.in_orig = h->orig;
   p.out = soa_of(h->A);
   p.out_key = h->keys;
-  p.flags = dsmcb::kDoFixup | dsmcb::kDoCollide | dsmcb::kDoMove | dsmcb::kDoKeys | dsmcb::kPadded;
+  p.flags = dsmcb::kDoFixup | dsmcb::kDoCollide | dsmcb::kDoMove | dsmcb::kDoKeys;
   if (h->cfg.sample_every > 0) p.flags |= dsmcb::kDoSample;
   p.cell_variant = h->variant;
   p.defer_list = h->orig;
@@ -1847,22 +1847,18 @@ int dsmc_stage_sort(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t nkeys,
     return DSMC_ERR_ARG;
   }
   char* w = (char*)workspace;
-  uint32_t tiles = (nkeys + dsmcb::kScanTile - 1) / dsmcb::kScanTile;
+  const uint32_t tiles = (nkeys + dsmcb::kScanTile - 1) / dsmcb::kScanTile;
+  // counts, scan-tile sums and counters first: one region to zero
   uint32_t* count = (uint32_t*)w; w += align256(4ull * (nkeys + 1));
-  uint32_t* start = (uint32_t*)w; w += align256(4ull * (nkeys + 1));
   uint32_t* tsum = (uint32_t*)w; w += align256(4ull * tiles);
-  uint32_t* ticket = (uint32_t*)w; w += align256(4ull * n);
-  uint32_t* tval = (uint32_t*)w; w += align256(4ull * n);
-  uint32_t* tpos = (uint32_t*)w; w += align256(4ull * n);
-  Meta* meta = (Meta*)w;
-  cudaError_t e = cudaMemsetAsync(count, 0, 4ull * (nkeys + 1), s);
-  if (!e) e = cudaMemsetAsync(tsum, 0, 4ull * tiles, s);
-  if (!e) e = cudaMemsetAsync(meta, 0, sizeof(Meta), s);
-  if (!e && n) e = dsmcb::launch_count_keys(keys, n, nkeys, ticket, count, tsum, tiles, s);
-  if (!e) e = dsmcb::launch_scan(count, nullptr, start, nkeys, tsum, tiles, meta, 0, s);
-  if (!e && n) e = dsmcb::launch_scatter_kv(keys, vals, ticket, start, n, nkeys, tval, tpos, s);
-  if (!e && n) e = dsmcb::launch_segment_fixup(start, nkeys, tval, tpos, keys, vals, s);
-  if (!e && cell_start) e = cudaMemcpyAsync(cell_start, start, 4ull * (nkeys + 1), cudaMemcpyDeviceToDevice, s);
+  Meta* meta = (Meta*)(((uintptr_t)w + 7u) & ~(uintptr_t)7u);  // (the workspace may start on 4 bytes)
+  w += align256(sizeof(Meta) + 8);
+  const size_t zeroed = (size_t)(w - (char*)workspace);
+  // the starts go straight to the caller when asked for
+  uint32_t* start = cell_start ? cell_start : (uint32_t*)w;
+  w += align256(4ull * (nkeys + 1));
+  cudaError_t e = cudaMemsetAsync(workspace, 0, zeroed, s);
+  if (!e) e = dsmcb::launch_sort(keys, vals, n, nkeys, count, start, tsum, (uint32_t*)w, meta, s);
   if (own) cudaFreeAsync(workspace, s);
   return e ? DSMC_ERR_CUDA : DSMC_OK;
 }
@@ -1883,7 +1879,7 @@ int dsmc_stage_collide(const dsmc_collide_params* cp, float* u, float* v, float*
                        void* stream) {
   if (!cp || !u || !v || !w || !cell_start || !maxrem) return DSMC_ERR_ARG;
   if (cp->rng == DSMC_RNG_TAUS && !seeds) return DSMC_ERR_ARG;
-  // the bulk copies of the kernel start on 16-byte boundaries of each array
+  // 16-byte boundaries of each array
   for (const void* a : {(const void*)u, (const void*)v, (const void*)w, (const void*)cell_start,
                         (const void*)maxrem, (const void*)seeds})
     if ((uintptr_t)a & 15u) return DSMC_ERR_ARG;
@@ -1909,12 +1905,9 @@ int dsmc_stage_collide(const dsmc_collide_params* cp, float* u, float* v, float*
   p.seeds = (uint4*)seeds;
   p.stat4 = (float4*)stat4;
   p.meta = nullptr;
-  p.flags = dsmcb::kDoCollide | dsmcb::kVelOnly;
-  p.cells_per_tile = 256;
-  p.n_tiles = (cp->ncells + 255) / 256;
+  p.flags = dsmcb::kDoCollide;
   p.step_override = cp->step ? cp->step : 1u;
-  p.cell_variant = 0;
-  cudaError_t e = dsmcb::launch_cell(p, (cudaStream_t)stream);
+  cudaError_t e = dsmcb::launch_collide_cells(p, (cudaStream_t)stream);
   return e ? DSMC_ERR_CUDA : DSMC_OK;
 }
 

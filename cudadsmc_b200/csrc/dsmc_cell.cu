@@ -108,19 +108,16 @@ __device__ Chunk make_chunk(const CellSmem<CAP>& S, uint32_t tile, int lsb, uint
 
 __device__ __forceinline__ bool chunk_has_data(const Chunk& c) { return !c.giant && c.n > 0; }
 
-// Element ranges of a chunk's copies.  Padded (the library's own buffers,
-// allocated with 16 bytes of slack): the whole 16-byte aligned cover of the
-// range.  Otherwise only the aligned interior; the ragged head and tail are
-// read with plain loads after the copy (ragged_chunk), so a caller's buffer is
-// never read past its end.
+// Element ranges of a chunk's copies: the whole 16-byte aligned cover of the
+// range (the library's buffers are allocated with 16 bytes of slack).
 struct Span {
   uint32_t ia, ib;
 };
-__device__ __forceinline__ Span span4(uint32_t b, uint32_t e, bool padded) {
-  return padded ? Span{b & ~3u, (e + 3u) & ~3u} : Span{(b + 3u) & ~3u, e & ~3u};
+__device__ __forceinline__ Span span4(uint32_t b, uint32_t e) {
+  return Span{b & ~3u, (e + 3u) & ~3u};
 }
-__device__ __forceinline__ Span span8(uint32_t b, uint32_t e, bool padded) {
-  return padded ? Span{b & ~1u, (e + 1u) & ~1u} : Span{(b + 1u) & ~1u, e & ~1u};
+__device__ __forceinline__ Span span8(uint32_t b, uint32_t e) {
+  return Span{b & ~1u, (e + 1u) & ~1u};
 }
 
 __device__ __forceinline__ const float* part_src(const StepParams& p, int a) {
@@ -140,26 +137,23 @@ __device__ __forceinline__ const float* part_src(const StepParams& p, int a) {
 template <int CAP>
 __device__ void issue_chunk(const StepParams& p, CellSmem<CAP>& S, const Chunk& c) {
   const unsigned lane = lane_id();
-  const bool padded = (p.flags & kPadded) != 0;
-  const bool vel_only = (p.flags & kVelOnly) != 0;
   const bool fix = (p.flags & kDoFixup) != 0;
   const bool collide = (p.flags & kDoCollide) != 0;
   const bool taus = p.rng_kind == 0;
   const uint32_t a0 = c.base & ~3u;
-  const Span ps = span4(c.base, c.base + c.n, padded);
+  const Span ps = span4(c.base, c.base + c.n);
   const uint32_t pbytes = ps.ib > ps.ia ? (ps.ib - ps.ia) * 4u : 0u;
   const uint32_t cs = c.c0 + c.cur;
-  const Span ms = span8(cs, cs + c.k, padded);
+  const Span ms = span8(cs, cs + c.k);
   const uint32_t mbytes = (collide && ms.ib > ms.ia) ? (ms.ib - ms.ia) * 8u : 0u;
   const uint32_t sbytes = (collide && taus) ? c.k * 16u : 0u;
-  const uint32_t narr = vel_only ? 3u : (fix ? 7u : 6u);
+  const uint32_t narr = fix ? 7u : 6u;
   unsigned long long* m = &S.mbar[c.buf];
   if (lane == 0) mbar_expect_tx(m, pbytes * narr + mbytes + sbytes);
   __syncwarp();
   fence_proxy_async();
-  const int first = vel_only ? 3 : 0;
   if (lane < narr) {
-    const int a = first + (int)lane;
+    const int a = (int)lane;
     if (pbytes) bulk_g2s(S.part[c.buf][a] + (ps.ia - a0), part_src(p, a) + ps.ia, pbytes, m);
   } else if (lane == 8 && mbytes) {
     bulk_g2s(S.maxrem[c.buf] + (ms.ia - (cs & ~1u)), p.maxrem + ms.ia, mbytes, m);
@@ -168,53 +162,16 @@ __device__ void issue_chunk(const StepParams& p, CellSmem<CAP>& S, const Chunk& 
   }
 }
 
-// The ragged ends of a chunk's copies (not padded), by plain loads.
-template <int CAP>
-__device__ void ragged_chunk(const StepParams& p, CellSmem<CAP>& S, const Chunk& c) {
-  const bool vel_only = (p.flags & kVelOnly) != 0;
-  const bool fix = (p.flags & kDoFixup) != 0;
-  const uint32_t a0 = c.base & ~3u, e = c.base + c.n;
-  const Span ps = span4(c.base, e, false);
-  const uint32_t narr = vel_only ? 3u : (fix ? 7u : 6u);
-  const int first = vel_only ? 3 : 0;
-  // head [base, min(ia, e)) and tail [max(ib, ia, base), e): at most 3 each
-  const uint32_t h1 = min(ps.ia, e), t0 = max(max(ps.ib, ps.ia), c.base);
-  for (uint32_t w = threadIdx.x; w < narr * 8u; w += blockDim.x) {
-    const int a = first + (int)(w >> 3);
-    const uint32_t r = w & 7u;
-    uint32_t i = kNone;
-    if (r < 4u) { if (c.base + r < h1) i = c.base + r; }
-    else if (t0 + (r - 4u) < e) i = t0 + (r - 4u);
-    if (i != kNone) S.part[c.buf][a][i - a0] = part_src(p, a)[i];
-  }
-  if ((p.flags & kDoCollide) && threadIdx.x == blockDim.x - 1) {
-    const uint32_t cs = c.c0 + c.cur, ce = cs + c.k;
-    const Span ms = span8(cs, ce, false);
-    for (uint32_t i = cs; i < min(ms.ia, ce); i++) S.maxrem[c.buf][i - (cs & ~1u)] = p.maxrem[i];
-    for (uint32_t i = max(max(ms.ib, ms.ia), cs); i < ce; i++)
-      S.maxrem[c.buf][i - (cs & ~1u)] = p.maxrem[i];
-  }
-}
-
-// Issues the copy of the cell starts of `tile` into ls buffer b (thread 0);
-// when not padded the ragged tail is read by finish_ls after the wait.
+// Issues the copy of the cell starts of `tile` into ls buffer b (thread 0).
 template <int CAP>
 __device__ void issue_ls(const StepParams& p, CellSmem<CAP>& S, uint32_t tile, int b) {
   const uint32_t ct = (uint32_t)p.cells_per_tile;
   const uint32_t nct = min(ct, p.cells - tile * ct);
-  const uint32_t whole = (p.flags & kPadded) ? ((nct + 1u + 3u) & ~3u) : ((nct + 1u) & ~3u);
+  const uint32_t whole = (nct + 1u + 3u) & ~3u;
   fence_proxy_async();
   mbar_expect_tx(&S.mbar_ls[b], whole * 4u);
-  if (whole) bulk_g2s(S.ls[b], p.start + tile * ct, whole * 4u, &S.mbar_ls[b]);
+  bulk_g2s(S.ls[b], p.start + tile * ct, whole * 4u, &S.mbar_ls[b]);
 }
-template <int CAP>
-__device__ void finish_ls(const StepParams& p, CellSmem<CAP>& S, uint32_t tile, int b) {
-  if (p.flags & kPadded) return;
-  const uint32_t ct = (uint32_t)p.cells_per_tile;
-  const uint32_t nct = min(ct, p.cells - tile * ct);
-  for (uint32_t i = (nct + 1u) & ~3u; i <= nct; i++) S.ls[b][i] = p.start[tile * ct + i];
-}
-
 // ----------------------------------------------------------- giant cell ----
 
 // A cell too large for the shared-memory chunk: processed by the whole block
@@ -224,7 +181,6 @@ static __device__ __noinline__ void giant_cell(const StepParams& p, uint32_t cel
                            uint32_t& col, double& sum_g, uint32_t& removed) {
   __shared__ double red[4][32];
   const uint32_t n = e - s;
-  const bool vel_only = (p.flags & kVelOnly) != 0;
   if (threadIdx.x == 0 && p.meta) atomicAdd(&p.meta->giant_cells, 1u);
   if (p.flags & kDoFixup) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -235,16 +191,12 @@ static __device__ __noinline__ void giant_cell(const StepParams& p, uint32_t cel
         rank += (o < my) | ((o == my) & (j < i));
       }
       const uint32_t d = s + rank;
-      if (!vel_only) {
-        p.out.x[d] = p.in.x[s + i]; p.out.y[d] = p.in.y[s + i]; p.out.z[d] = p.in.z[s + i];
-      }
+      p.out.x[d] = p.in.x[s + i]; p.out.y[d] = p.in.y[s + i]; p.out.z[d] = p.in.z[s + i];
       p.out.u[d] = p.in.u[s + i]; p.out.v[d] = p.in.v[s + i]; p.out.w[d] = p.in.w[s + i];
     }
   } else if (p.out.u != p.in.u) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      if (!vel_only) {
-        p.out.x[s + i] = p.in.x[s + i]; p.out.y[s + i] = p.in.y[s + i]; p.out.z[s + i] = p.in.z[s + i];
-      }
+      p.out.x[s + i] = p.in.x[s + i]; p.out.y[s + i] = p.in.y[s + i]; p.out.z[s + i] = p.in.z[s + i];
       p.out.u[s + i] = p.in.u[s + i]; p.out.v[s + i] = p.in.v[s + i]; p.out.w[s + i] = p.in.w[s + i];
     }
   }
@@ -266,7 +218,7 @@ static __device__ __noinline__ void giant_cell(const StepParams& p, uint32_t cel
     bool live = true;
     if (active) {
       const uint32_t g = s + q;
-      if (!vel_only) pos = make_float3(p.out.x[g], p.out.y[g], p.out.z[g]);
+      pos = make_float3(p.out.x[g], p.out.y[g], p.out.z[g]);
       vel = make_float3(p.out.u[g], p.out.v[g], p.out.w[g]);
       if (p.flags & kDoMove) live = move_particle(p, pos, vel, g, step);
       if (do_sample) {
@@ -274,7 +226,7 @@ static __device__ __noinline__ void giant_cell(const StepParams& p, uint32_t cel
         su += x; sv += y; sw += z;
         se += x * x + y * y + z * z;
       }
-      if (!vel_only) { p.out.x[g] = pos.x; p.out.y[g] = pos.y; p.out.z[g] = pos.z; }
+      p.out.x[g] = pos.x; p.out.y[g] = pos.y; p.out.z[g] = pos.z;
       p.out.u[g] = vel.x; p.out.v[g] = vel.y; p.out.w[g] = vel.z;
     }
     if (p.flags & kDoKeys) {
@@ -327,8 +279,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_cell(const __grid_constant__ 
   const bool do_fixup = (p.flags & kDoFixup) != 0;
   const bool do_collide = (p.flags & kDoCollide) != 0;
   const bool do_keys = (p.flags & kDoKeys) != 0;
-  const bool vel_only = (p.flags & kVelOnly) != 0;
-  const bool padded = (p.flags & kPadded) != 0;
   const bool taus = p.rng_kind == 0;
   const bool heavy_mode = !taus && do_collide;
   const uint32_t ct = (uint32_t)p.cells_per_tile;
@@ -365,7 +315,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_cell(const __grid_constant__ 
   }
   if (warp == 0 && blockIdx.x < p.n_tiles) {
     if (tid == 0) {
-      finish_ls(p, S, blockIdx.x, 0);
       S.cur = make_chunk(S, blockIdx.x, 0, 0, ct, p.cells, 0);
       S.cur.ntile = tiles.grab(p);
       pending = tiles.grab(p);
@@ -413,7 +362,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_cell(const __grid_constant__ 
           nx = make_chunk(S, c.tile, c.lsb, c.cur + c.k, ct, p.cells, 1 - c.buf);
           nx.ntile = nt;
         } else if (nt < p.n_tiles) {
-          finish_ls(p, S, nt, nb);
           nx = make_chunk(S, nt, nb, 0, ct, p.cells, 1 - c.buf);
           nx.ntile = pending;
           pending = tiles.grab(p);
@@ -425,10 +373,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_cell(const __grid_constant__ 
       }
       __syncwarp();
       if (S.next.valid && chunk_has_data(S.next)) issue_chunk(p, S, S.next);
-    }
-    if (chunk_has_data(c) && !padded) {
-      ragged_chunk(p, S, c);
-      __syncthreads();
     }
     const uint32_t* ls = S.ls[c.lsb];
     if (c.giant) {
@@ -521,7 +465,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_cell(const __grid_constant__ 
           if (active) {
             q = pass == 0 ? i : (uint32_t)S.hardq[i];
             j = S.slot[q];
-            if (!vel_only) pos = make_float3(X[j], Y[j], Z[j]);
+            pos = make_float3(X[j], Y[j], Z[j]);
             vel = make_float3(U[j], V[j], W[j]);
             if (pass == 0 && split) defer = flight_may_meet_body(p, pos, vel);
           }
@@ -541,7 +485,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_cell(const __grid_constant__ 
             if (p.flags & kDoMove)
               live = pass == 0 ? move_free(p, pos, vel, g, step) : move_particle(p, pos, vel, g, step);
             if (do_sample) { U[j] = vel.x; V[j] = vel.y; W[j] = vel.z; }
-            if (!vel_only) { p.out.x[g] = pos.x; p.out.y[g] = pos.y; p.out.z[g] = pos.z; }
+            p.out.x[g] = pos.x; p.out.y[g] = pos.y; p.out.z[g] = pos.z;
             p.out.u[g] = vel.x; p.out.v[g] = vel.y; p.out.w[g] = vel.z;
           }
           if (do_keys) {
@@ -626,8 +570,7 @@ cudaError_t launch_variant(const StepParams& p, cudaStream_t stream) {
 }  // namespace
 
 // Variants 0-3: the CTA-wide kernel above; 4-7: the warp-autonomous kernel
-// (dsmc_cellw.cu), which handles the full step with padded buffers (the
-// collide stage, kVelOnly on caller buffers, always runs the CTA-wide one).
+// (dsmc_cellw.cu).
 int cell_kernel_variants() { return 4 + cell_kernel_w_variants(); }
 
 int cell_kernel_chunk_capacity(int variant) {
@@ -639,7 +582,7 @@ int cell_kernel_chunk_capacity(int variant) {
 bool cell_kernel_is_warp(int variant) { return variant >= 4; }
 
 cudaError_t launch_cell(const StepParams& p, cudaStream_t stream) {
-  if (p.cell_variant >= 4 && (p.flags & kPadded) && !(p.flags & kVelOnly))
+  if (p.cell_variant >= 4)
     return launch_cell_w(p, p.cell_variant - 4, stream);
   switch (p.cell_variant) {
     case 0: return launch_variant<512, 2048, 1>(p, stream);

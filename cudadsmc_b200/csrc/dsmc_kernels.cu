@@ -18,15 +18,31 @@ namespace {
 
 using namespace dev;
 
-// Move stage: free flight and boundaries for n particles in place.
+// Move stage: free flight and boundaries for n particles in place.  Without a
+// body each thread flies four at a time, their loads in flight together (4.2M
+// particles: 50 -> 28 us).
+template <bool BODY>
 __global__ void __launch_bounds__(256) k_move(const __grid_constant__ StepParams p, uint32_t n, uint32_t step) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float3 pos = make_float3(p.out.x[i], p.out.y[i], p.out.z[i]);
-    float3 vel = make_float3(p.out.u[i], p.out.v[i], p.out.w[i]);
-    const bool live = move_particle(p, pos, vel, i, step);
-    p.out.x[i] = live ? pos.x : __int_as_float(0x7fc00000);
-    p.out.y[i] = pos.y; p.out.z[i] = pos.z;
-    p.out.u[i] = vel.x; p.out.v[i] = vel.y; p.out.w[i] = vel.z;
+  constexpr int U = BODY ? 1 : 4;
+  for (uint32_t base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+    float3 pos[U], vel[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      if (i < n) {
+        pos[k] = make_float3(p.out.x[i], p.out.y[i], p.out.z[i]);
+        vel[k] = make_float3(p.out.u[i], p.out.v[i], p.out.w[i]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      if (i >= n) continue;
+      const bool live = BODY ? move_particle(p, pos[k], vel[k], i, step) : move_free(p, pos[k], vel[k], i, step);
+      p.out.x[i] = live ? pos[k].x : __int_as_float(0x7fc00000);
+      p.out.y[i] = pos[k].y; p.out.z[i] = pos[k].z;
+      p.out.u[i] = vel[k].x; p.out.v[i] = vel[k].y; p.out.w[i] = vel[k].z;
+    }
   }
 }
 
@@ -35,9 +51,21 @@ __global__ void __launch_bounds__(256) k_cell_ids(GridGeom g, const float* __res
                                                   const float* __restrict__ z, uint32_t n,
                                                   uint32_t* __restrict__ keys,
                                                   uint32_t* __restrict__ idx) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    keys[i] = cell_id3d(g, x[i], y[i], z[i]);
-    if (idx) idx[i] = i;
+  constexpr int U = 4;  // positions in flight per thread
+  for (uint32_t base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+    float3 q[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      if (i < n) q[k] = make_float3(x[i], y[i], z[i]);
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      if (i >= n) continue;
+      keys[i] = cell_id3d(g, q[k].x, q[k].y, q[k].z);
+      if (idx) idx[i] = i;
+    }
   }
 }
 
@@ -280,57 +308,109 @@ __global__ void __launch_bounds__(256, 4) k_scatter_b(const __grid_constant__ Ba
 
 // ------------------------------------------------------------ sort stage ----
 
+// A counting sort: counts per key, their scan, each entry to its key's range
+// in any order (a ticket from the key's count, which the scan left at zero),
+// and the input order restored inside each key.  Counting without tickets
+// (non-returning atomics) and taking them in the scatter, four groups of 32
+// in flight per warp, costs less than storing them: 4.2M entries, 524,288
+// keys: count and scatter 45 + 27 -> 19 + 35 us.
 // Keys >= nkeys are left out of the sort (no ticket, no slot).
-__global__ void k_count_keys(const uint32_t* __restrict__ keys, uint32_t n, uint32_t nkeys,
-                             uint32_t* __restrict__ ticket, uint32_t* count, uint32_t* tile_sum,
-                             uint32_t n_scan_tiles) {
+__global__ void __launch_bounds__(256) k_count_keys(const uint32_t* __restrict__ keys, uint32_t n, uint32_t nkeys,
+                                                    uint32_t* count, uint32_t* tile_sum, uint32_t n_scan_tiles) {
   extern __shared__ uint32_t s_tile[];
   for (uint32_t t = threadIdx.x; t < n_scan_tiles; t += blockDim.x) s_tile[t] = 0;
   __syncthreads();
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t key = i < n ? keys[i] : kNone;
-    const bool active = i < n && key < nkeys;
-    const unsigned m = __ballot_sync(kFull, active);
-    if (active) {
-      const uint32_t t = warp_ticket(count, key, m);
-      ticket[i] = t;
-      const unsigned peers = __match_any_sync(m, key);
-      if ((int)lane_id() == __ffs(peers) - 1) atomicAdd(&s_tile[key >> kScanShift], (uint32_t)__popc(peers));
+  constexpr int U = 4;
+  for (uint32_t base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+    uint32_t key[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      key[k] = i < n ? keys[i] : kNone;
     }
+#pragma unroll
+    for (int k = 0; k < U; k++)
+      if (key[k] < nkeys) warp_count_key(count, key[k], 0u, s_tile);
   }
   __syncthreads();
   flush_tile_hist(s_tile, tile_sum, n_scan_tiles);
 }
 
-__global__ void k_scatter_kv(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
-                             const uint32_t* __restrict__ ticket,
-                             const uint32_t* __restrict__ start, uint32_t n, uint32_t nkeys,
-                             uint32_t* __restrict__ tmp_val, uint32_t* __restrict__ tmp_pos) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t key = keys[i];
-    if (key >= nkeys) continue;
-    const uint32_t d = start[key] + ticket[i];
-    tmp_val[d] = vals[i];
-    tmp_pos[d] = i;
+// Where the scatter puts (value, input position) of an entry: pairs where the
+// workspace is 8-byte aligned (one store, one sector), else two arrays.
+template <bool PAIR>
+struct ScatterOut {
+  uint32_t* val;
+  uint32_t* pos;
+  __device__ __forceinline__ void put(uint32_t d, uint32_t v, uint32_t i) const {
+    if (PAIR) {
+      reinterpret_cast<uint2*>(val)[d] = make_uint2(v, i);
+    } else {
+      val[d] = v;
+      pos[d] = i;
+    }
+  }
+  __device__ __forceinline__ uint2 get(uint32_t d) const {
+    return PAIR ? reinterpret_cast<const uint2*>(val)[d] : make_uint2(val[d], pos[d]);
+  }
+};
+
+template <bool PAIR>
+__global__ void __launch_bounds__(256) k_scatter_kv(const uint32_t* __restrict__ keys,
+                                                    const uint32_t* __restrict__ vals,
+                                                    const uint32_t* __restrict__ start, uint32_t* cursor, uint32_t n,
+                                                    uint32_t nkeys, ScatterOut<PAIR> out) {
+  constexpr int U = 4;
+  const uint32_t lane = lane_id();
+  for (uint32_t base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+    uint32_t key[U], val[U], st[U], got[U];
+    unsigned peers[U], msk[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      key[k] = i < n ? keys[i] : kNone;
+      val[k] = i < n ? vals[i] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const bool live = key[k] < nkeys;
+      msk[k] = __ballot_sync(kFull, live);
+      st[k] = got[k] = 0;
+      peers[k] = 0;
+      if (live) {
+        st[k] = __ldg(&start[key[k]]);
+        peers[k] = __match_any_sync(msk[k], key[k]);
+        if ((int)lane == __ffs(peers[k]) - 1) got[k] = atomicAdd(&cursor[key[k]], (uint32_t)__popc(peers[k]));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      if (!(key[k] < nkeys)) continue;
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      const uint32_t t = __shfl_sync(msk[k], got[k], __ffs(peers[k]) - 1) + __popc(peers[k] & ((1u << lane) - 1u));
+      out.put(st[k] + t, val[k], i);
+    }
   }
 }
 
 // Restores input order within each key: entry of rank r (by input position)
-// among its key's entries goes to start[key] + r.
-__global__ void __launch_bounds__(256) k_segment_fixup(const uint32_t* __restrict__ start,
-                                                       uint32_t nkeys,
-                                                       const uint32_t* __restrict__ tmp_val,
-                                                       const uint32_t* __restrict__ tmp_pos,
-                                                       uint32_t* __restrict__ keys_out,
-                                                       uint32_t* __restrict__ vals_out) {
-  constexpr int kCap = 4096;
-  __shared__ uint32_t ls[257];
-  __shared__ uint32_t spos[kCap];
-  __shared__ uint32_t sval[kCap];
-  const uint32_t ntiles = (nkeys + 255) / 256;
+// among its key's entries goes to start[key] + r.  A CTA takes kt keys at a
+// time (at most kFixupThreads), in chunks of whole keys of at most kFixupCap
+// entries in shared memory; tiles are small (launch_segment_fixup), so that a
+// few thousand keys reach every SM (4,096 keys of 24: 35 us with tiles of 256
+// keys on 16 CTAs, now 5 us; 524,288 keys of 8: 58, now 34 us).
+constexpr int kFixupThreads = 128, kFixupCap = 1024;
+template <bool PAIR>
+__global__ void __launch_bounds__(kFixupThreads) k_segment_fixup(const uint32_t* __restrict__ start, uint32_t nkeys,
+                                                                 uint32_t kt, ScatterOut<PAIR> in,
+                                                                 uint32_t* __restrict__ keys_out,
+                                                                 uint32_t* __restrict__ vals_out) {
+  __shared__ uint32_t ls[kFixupThreads + 1];
+  __shared__ uint32_t spos[kFixupCap];
+  __shared__ uint8_t cellof[kFixupCap];  // the chunk's key of each entry
+  const uint32_t ntiles = (nkeys + kt - 1) / kt;
   for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint32_t c0 = tile * 256, nct = min(256u, nkeys - c0);
+    const uint32_t c0 = tile * kt, nct = min(kt, nkeys - c0);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i <= nct; i += blockDim.x) ls[i] = start[c0 + i];
     __syncthreads();
@@ -338,40 +418,48 @@ __global__ void __launch_bounds__(256) k_segment_fixup(const uint32_t* __restric
     while (cur < nct) {
       const uint32_t base = ls[cur];
       const uint32_t c = cur + 1 + threadIdx.x;
-      const int fits = (c <= nct) && (ls[c] - base <= (uint32_t)kCap);
+      const int fits = (c <= nct) && (ls[c] - base <= (uint32_t)kFixupCap);
       const uint32_t k = __syncthreads_count(fits);
       if (k == 0) {
-        // one key with more than kCap entries: rank from global memory
+        // one key with more than kFixupCap entries: rank from global memory
         const uint32_t s0 = base, e0 = ls[cur + 1];
         for (uint32_t i = s0 + threadIdx.x; i < e0; i += blockDim.x) {
-          const uint32_t my = tmp_pos[i];
+          const uint2 my = in.get(i);
           uint32_t rank = 0;
-          for (uint32_t j = s0; j < e0; j++) rank += tmp_pos[j] < my;
+          for (uint32_t j = s0; j < e0; j++) rank += in.get(j).y < my.y;
           keys_out[s0 + rank] = c0 + cur;
-          vals_out[s0 + rank] = tmp_val[i];
+          vals_out[s0 + rank] = my.x;
         }
         cur += 1;
         __syncthreads();
         continue;
       }
       const uint32_t n = ls[cur + k] - base;
-      for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
-        spos[t] = tmp_pos[base + t];
-        sval[t] = tmp_val[base + t];
+      if (threadIdx.x < k)
+        for (uint32_t j = ls[cur + threadIdx.x]; j < ls[cur + threadIdx.x + 1]; j++)
+          cellof[j - base] = (uint8_t)threadIdx.x;
+      uint32_t val[kFixupCap / kFixupThreads];
+#pragma unroll
+      for (int q = 0; q < kFixupCap / kFixupThreads; q++) {
+        const uint32_t t = threadIdx.x + q * kFixupThreads;
+        if (t < n) {
+          const uint2 e = in.get(base + t);
+          val[q] = e.x;
+          spos[t] = e.y;
+        }
       }
       __syncthreads();
-      for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
-        uint32_t lo = cur, hi = cur + k - 1;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi + 1) >> 1;
-          if (ls[mid] - base <= t) lo = mid; else hi = mid - 1;
-        }
+#pragma unroll
+      for (int q = 0; q < kFixupCap / kFixupThreads; q++) {
+        const uint32_t t = threadIdx.x + q * kFixupThreads;
+        if (t >= n) break;
+        const uint32_t lo = cur + cellof[t];
         const uint32_t s0 = ls[lo] - base, e0 = ls[lo + 1] - base;
         const uint32_t my = spos[t];
         uint32_t rank = 0;
         for (uint32_t j = s0; j < e0; j++) rank += spos[j] < my;
         keys_out[base + s0 + rank] = c0 + lo;
-        vals_out[base + s0 + rank] = sval[t];
+        vals_out[base + s0 + rank] = val[q];
       }
       cur += k;
       __syncthreads();
@@ -381,26 +469,53 @@ __global__ void __launch_bounds__(256) k_segment_fixup(const uint32_t* __restric
 
 // FindCellBoundariesDev (kernels/dsmc_kernel.cu:1734-1787): start/end per
 // cell from sorted keys (cse zeroed by the caller) and the gather.
-__global__ void k_bounds_reorder(const uint32_t* __restrict__ keys,
-                                 const uint32_t* __restrict__ idx, uint32_t n, uint32_t ncells,
-                                 uint2* cse, SoA src, SoA dst, int gather) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t h = keys[i];
-    const uint32_t hp = i > 0 ? keys[i - 1] : kNone;
-    if (i == 0 || h != hp) {
-      if (h < ncells) cse[h].x = i;
-      if (i > 0 && hp < ncells) cse[hp].y = i;
+// Each thread gathers four particles at a time, their 24 loads in flight
+// together (4.2M particles: 66 -> 61 us, 3.8 TB/s: what is left is the gather's
+// sectors and the bounds' scattered words).
+__global__ void __launch_bounds__(256) k_bounds_reorder(const uint32_t* __restrict__ keys,
+                                                        const uint32_t* __restrict__ idx, uint32_t n, uint32_t ncells,
+                                                        uint2* cse, SoA src, SoA dst, int gather) {
+  constexpr int U = 4;
+  for (uint32_t base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
+    uint32_t s[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      s[k] = gather && i < n ? idx[i] : 0u;
     }
-    if (i == n - 1 && h < ncells) cse[h].y = i + 1;
-    if (gather) {
-      const uint32_t s = idx[i];
-      dst.x[i] = src.x[s]; dst.y[i] = src.y[s]; dst.z[i] = src.z[s];
-      dst.u[i] = src.u[s]; dst.v[i] = src.v[s]; dst.w[i] = src.w[s];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      if (i >= n) continue;
+      const uint32_t h = keys[i];
+      const uint32_t hp = i > 0 ? keys[i - 1] : kNone;
+      if (i == 0 || h != hp) {
+        if (h < ncells) cse[h].x = i;
+        if (i > 0 && hp < ncells) cse[hp].y = i;
+      }
+      if (i == n - 1 && h < ncells) cse[h].y = i + 1;
+    }
+    if (!gather) continue;
+    float v[6][U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      if (i >= n) continue;
+      v[0][k] = src.x[s[k]]; v[1][k] = src.y[s[k]]; v[2][k] = src.z[s[k]];
+      v[3][k] = src.u[s[k]]; v[4][k] = src.v[s[k]]; v[5][k] = src.w[s[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      if (i >= n) continue;
+      dst.x[i] = v[0][k]; dst.y[i] = v[1][k]; dst.z[i] = v[2][k];
+      dst.u[i] = v[3][k]; dst.v[i] = v[4][k]; dst.w[i] = v[5][k];
     }
   }
 }
 
-// Stand-alone FP64 sampling, one thread per cell.
+// Stand-alone FP64 sampling, one thread per cell, a cell's loads four
+// particles at a time and its sums in order.
 __global__ void k_sample_cells(const float* __restrict__ u, const float* __restrict__ v,
                                const float* __restrict__ w, const uint32_t* __restrict__ start,
                                uint32_t cells, double* acc, size_t fs, size_t cs) {
@@ -408,16 +523,94 @@ __global__ void k_sample_cells(const float* __restrict__ u, const float* __restr
     const uint32_t s = start[c], e = start[c + 1];
     if (e <= s) continue;
     double su = 0, sv = 0, sw = 0, se = 0;
-    for (uint32_t i = s; i < e; i++) {
-      const double x = u[i], y = v[i], z = w[i];
+    auto add = [&](float a, float b, float d) {
+      const double x = a, y = b, z = d;
       su += x; sv += y; sw += z;
       se += x * x + y * y + z * z;
+    };
+    uint32_t i = s;
+    for (; i + 4u <= e; i += 4u) {
+      const float x0 = u[i], x1 = u[i + 1], x2 = u[i + 2], x3 = u[i + 3];
+      const float y0 = v[i], y1 = v[i + 1], y2 = v[i + 2], y3 = v[i + 3];
+      const float z0 = w[i], z1 = w[i + 1], z2 = w[i + 2], z3 = w[i + 3];
+      add(x0, y0, z0);
+      add(x1, y1, z1);
+      add(x2, y2, z2);
+      add(x3, y3, z3);
     }
+    for (; i < e; i++) add(u[i], v[i], w[i]);
     acc[c * cs] += (double)(e - s);
     acc[fs + c * cs] += su;
     acc[2 * fs + c * cs] += sv;
     acc[3 * fs + c * cs] += sw;
     acc[4 * fs + c * cs] += se;
+  }
+}
+
+// Collide stage: the NTC collisions of every cell of the caller's sorted
+// velocities, in place.  A warp takes ct <= 32 consecutive cells, a lane each;
+// cells with many pairs (Philox mode) follow, the whole warp on each.  The
+// same draws and arithmetic per cell as the fused cell kernel in its
+// 2048-particle form, which this replaces here: that one staged a chunk of
+// cells per CTA between barriers, on 16 CTAs for 4,096 cells (4,096 cells of
+// 24: 34 -> 12 us; 524,288 of 8: 183 -> 36 us).
+constexpr int kCollideWarps = 8;
+constexpr uint32_t kCollideClaim = 256;    // largest cell staged in shared memory
+constexpr uint32_t kCollideGiant = 2048;   // above: one lane whatever its pairs
+__global__ void __launch_bounds__(32 * kCollideWarps) k_collide_cells(const __grid_constant__ StepParams p,
+                                                                      uint32_t ct) {
+  __shared__ uint32_t s_claim[kCollideWarps][kCollideClaim];
+  __shared__ float s_vel[kCollideWarps][3][kCollideClaim];
+  const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+  for (uint32_t t = lane; t < kCollideClaim; t += 32) s_claim[warp][t] = 0xffffffffu;
+  __syncwarp();
+  const bool taus = p.rng_kind == 0;
+  uint32_t sel = 0, col = 0;
+  double sum_g = 0.0;
+  const uint32_t tiles = (p.cells + ct - 1u) / ct;
+  for (uint32_t t = blockIdx.x * kCollideWarps + warp; t < tiles; t += gridDim.x * kCollideWarps) {
+    const uint32_t c = t * ct + lane;
+    const bool mine = lane < ct && c < p.cells;
+    uint32_t s = 0, n = 0;
+    bool heavy = false;
+    if (mine) {
+      s = p.start[c];
+      n = p.start[c + 1] - s;
+      if (!taus && n >= 2 && n <= kCollideGiant) heavy = (uint32_t)ntc_fpc_fast(p, n, p.maxrem[c]) >= kHeavyMin;
+    }
+    if (mine && !heavy) {
+      GlobalVel acc{p.in.u, p.in.v, p.in.w, s};
+      CellState st{p.maxrem + c, taus ? p.seeds + c : nullptr, p.stat4 ? p.stat4 + c : nullptr};
+      collide_cell(p, c, (int)n, acc, p.step_override, st, sel, col, sum_g);
+    }
+    __syncwarp();
+    for (unsigned m = __ballot_sync(kFull, heavy); m; m &= m - 1u) {
+      const int l = __ffs(m) - 1;
+      const uint32_t hc = t * ct + (uint32_t)l, hs = __shfl_sync(kFull, s, l), hn = __shfl_sync(kFull, n, l);
+      CellState st{p.maxrem + hc, nullptr, p.stat4 ? p.stat4 + hc : nullptr};
+      GlobalVel acc{p.in.u, p.in.v, p.in.w, hs};
+      if (hn > kCollideClaim) {
+        ntc_heavy_warp(p, hc, hn, acc, nullptr, p.step_override, st, sel, col, sum_g);
+      } else {
+        float* su = s_vel[warp][0];
+        float* sv = s_vel[warp][1];
+        float* sw = s_vel[warp][2];
+        for (uint32_t k = lane; k < hn; k += 32) {
+          su[k] = acc.u[hs + k];
+          sv[k] = acc.v[hs + k];
+          sw[k] = acc.w[hs + k];
+        }
+        __syncwarp();
+        ntc_heavy_warp(p, hc, hn, GlobalVel{su, sv, sw, 0u}, s_claim[warp], p.step_override, st, sel, col, sum_g);
+        __syncwarp();
+        for (uint32_t k = lane; k < hn; k += 32) {
+          acc.u[hs + k] = su[k];
+          acc.v[hs + k] = sv[k];
+          acc.w[hs + k] = sw[k];
+        }
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -692,43 +885,53 @@ cudaError_t launch_scatter(bool with_state, const SoA& src, SoA dst, const uint3
 
 cudaError_t launch_move(const StepParams& p, uint32_t n, uint32_t step, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
-  const uint32_t grid = grid_for(n, 256, 8);
-  k_move<<<grid, 256, 0, stream>>>(p, n, step);
+  if (p.has_geom) k_move<true><<<grid_for(n, 256, 8), 256, 0, stream>>>(p, n, step);
+  else k_move<false><<<grid_for(n, 1024, 8), 256, 0, stream>>>(p, n, step);
   return cudaGetLastError();
 }
 
 cudaError_t launch_cell_ids(const GridGeom& g, const float* x, const float* y, const float* z,
                             uint32_t n, uint32_t* keys, uint32_t* idx, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
-  const uint32_t grid = grid_for(n, 256, 8);
-  k_cell_ids<<<grid, 256, 0, stream>>>(g, x, y, z, n, keys, idx);
+  k_cell_ids<<<grid_for(n, 1024, 8), 256, 0, stream>>>(g, x, y, z, n, keys, idx);
   return cudaGetLastError();
 }
 
-cudaError_t launch_count_keys(const uint32_t* keys, uint32_t n, uint32_t nkeys, uint32_t* ticket,
-                              uint32_t* count, uint32_t* tile_sum, uint32_t n_scan_tiles,
-                              cudaStream_t stream) {
-  const uint32_t grid = grid_for(n, 256, 8);
-  k_count_keys<<<grid, 256, n_scan_tiles * 4, stream>>>(keys, n, nkeys, ticket, count, tile_sum,
-                                                        n_scan_tiles);
+cudaError_t launch_sort(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t nkeys, uint32_t* count,
+                        uint32_t* start, uint32_t* tile_sum, uint32_t* scratch, Meta* meta, cudaStream_t stream) {
+  const uint32_t tiles = (nkeys + kScanTile - 1) / kScanTile;
+  if (n) {
+    k_count_keys<<<grid_for(n, 1024, 8), 256, tiles * 4, stream>>>(keys, n, nkeys, count, tile_sum, tiles);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  cudaError_t e = launch_scan(count, nullptr, start, nkeys, tile_sum, tiles, meta, 0, stream);
+  if (e != cudaSuccess || !n) return e;
+  // keys per CTA of the fixup: 64 where that makes eight tiles per SM, down to
+  // 8 on small key ranges
+  uint32_t kt = 64;
+  while (kt > 8 && nkeys / kt < (uint32_t)num_sms() * 8u) kt >>= 1;
+  const uint32_t ft = (nkeys + kt - 1) / kt, fgrid = std::min(ft, (uint32_t)num_sms() * 16u);
+  const uint32_t sgrid = grid_for(n, 1024, 8);
+  if (((uintptr_t)scratch & 7u) == 0) {
+    const ScatterOut<true> o{scratch, nullptr};
+    k_scatter_kv<true><<<sgrid, 256, 0, stream>>>(keys, vals, start, count, n, nkeys, o);
+    k_segment_fixup<true><<<fgrid, kFixupThreads, 0, stream>>>(start, nkeys, kt, o, keys, vals);
+  } else {
+    const ScatterOut<false> o{scratch, scratch + n};
+    k_scatter_kv<false><<<sgrid, 256, 0, stream>>>(keys, vals, start, count, n, nkeys, o);
+    k_segment_fixup<false><<<fgrid, kFixupThreads, 0, stream>>>(start, nkeys, kt, o, keys, vals);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_scatter_kv(const uint32_t* keys, const uint32_t* vals, const uint32_t* ticket,
-                              const uint32_t* start, uint32_t n, uint32_t nkeys, uint32_t* tmp_val,
-                              uint32_t* tmp_pos, cudaStream_t stream) {
-  const uint32_t grid = grid_for(n, 256, 8);
-  k_scatter_kv<<<grid, 256, 0, stream>>>(keys, vals, ticket, start, n, nkeys, tmp_val, tmp_pos);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_segment_fixup(const uint32_t* start, uint32_t nkeys, const uint32_t* tmp_val,
-                                 const uint32_t* tmp_pos, uint32_t* keys_out, uint32_t* vals_out,
-                                 cudaStream_t stream) {
-  const uint32_t ntiles = (nkeys + 255) / 256;
-  const uint32_t grid = ntiles < (uint32_t)num_sms() * 4 ? ntiles : (uint32_t)num_sms() * 4;
-  if (grid == 0) return cudaSuccess;
-  k_segment_fixup<<<grid, 256, 0, stream>>>(start, nkeys, tmp_val, tmp_pos, keys_out, vals_out);
+cudaError_t launch_collide_cells(const StepParams& p, cudaStream_t stream) {
+  if (p.cells == 0) return cudaSuccess;
+  // 32 cells per warp where that makes a wave of warps, fewer on small grids
+  uint32_t ct = 32;
+  while (ct > 1 && p.cells / ct < (uint32_t)num_sms() * 16u) ct >>= 1;
+  const uint32_t tiles = (p.cells + ct - 1) / ct;
+  k_collide_cells<<<grid_for(tiles, kCollideWarps, 8), 32 * kCollideWarps, 0, stream>>>(p, ct);
   return cudaGetLastError();
 }
 
@@ -740,7 +943,7 @@ cudaError_t launch_bounds_reorder(const uint32_t* keys, const uint32_t* idx, uin
         const_cast<float*>(src ? src[4] : nullptr), const_cast<float*>(src ? src[5] : nullptr)};
   SoA d{dst ? dst[0] : nullptr, dst ? dst[1] : nullptr, dst ? dst[2] : nullptr,
         dst ? dst[3] : nullptr, dst ? dst[4] : nullptr, dst ? dst[5] : nullptr};
-  const uint32_t grid = grid_for(n, 256, 8);
+  const uint32_t grid = grid_for(n, 1024, 8);
   k_bounds_reorder<<<grid, 256, 0, stream>>>(keys, idx, n, ncells, (uint2*)cse, s, d,
                                              (src && dst) ? 1 : 0);
   return cudaGetLastError();
@@ -756,8 +959,8 @@ cudaError_t launch_cell_fields(const double* acc, uint32_t cells, double fnum, d
 cudaError_t launch_sample_cells(const float* u, const float* v, const float* w,
                                 const uint32_t* start, uint32_t cells, double* acc,
                                 size_t fstride, size_t cstride, cudaStream_t stream) {
-  const uint32_t grid = grid_for(cells, 256, 8);
-  k_sample_cells<<<grid, 256, 0, stream>>>(u, v, w, start, cells, acc, fstride, cstride);
+  const uint32_t grid = grid_for(cells, 64, 32);  // small blocks: a few thousand cells reach every SM
+  k_sample_cells<<<grid, 64, 0, stream>>>(u, v, w, start, cells, acc, fstride, cstride);
   return cudaGetLastError();
 }
 

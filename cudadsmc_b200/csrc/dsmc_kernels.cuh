@@ -89,8 +89,6 @@ enum : int {
   kDoKeys = 8,     // next-step key + count + tile histogram
   kDoSample = 16,  // FP64 sampling after the move (every sample_every steps)
   kSampleForce = 32,  // sample regardless of the step counter
-  kVelOnly = 64,      // stage only velocities (collide stage)
-  kPadded = 128,      // buffers carry 16 bytes of slack: whole aligned copies
 };
 
 // Inflow description for a face that injects (extension).
@@ -207,7 +205,8 @@ cudaError_t launch_scatter(bool with_state, const SoA& src, SoA dst, const uint3
                            uint32_t* cursor, uint32_t* orig, uint32_t cells, uint32_t* tile_sum,
                            uint32_t n_scan_tiles, Meta* meta, uint32_t capacity,
                            cudaStream_t stream);
-// The timestep's fused cell kernel (also the collide stage with kVelOnly).
+// The timestep's cell kernels (fused or split); the buffers carry 16 bytes of
+// slack, so that bulk copies take whole aligned ranges.
 cudaError_t launch_cell(const StepParams& p, cudaStream_t stream);
 // Variants of the cell kernel.  CTA-wide: 0 (512 threads, 2048 particles per
 // chunk, 1 CTA/SM), 1 (256, 1024, 2), 2 (128, 512, 4), 3 (64, 256, up to 8).
@@ -233,16 +232,14 @@ cudaError_t launch_move(const StepParams& p, uint32_t n, uint32_t step, cudaStre
 cudaError_t launch_cell_ids(const GridGeom& g, const float* x, const float* y, const float* z,
                             uint32_t n, uint32_t* keys, uint32_t* idx, cudaStream_t stream);
 
-// Sort stage pieces (dsmc_stage_sort).
-cudaError_t launch_count_keys(const uint32_t* keys, uint32_t n, uint32_t nkeys, uint32_t* ticket,
-                              uint32_t* count, uint32_t* tile_sum, uint32_t n_scan_tiles,
-                              cudaStream_t stream);
-cudaError_t launch_scatter_kv(const uint32_t* keys, const uint32_t* vals, const uint32_t* ticket,
-                              const uint32_t* start, uint32_t n, uint32_t nkeys, uint32_t* tmp_val,
-                              uint32_t* tmp_pos, cudaStream_t stream);
-cudaError_t launch_segment_fixup(const uint32_t* start, uint32_t nkeys, const uint32_t* tmp_val,
-                                 const uint32_t* tmp_pos, uint32_t* keys_out, uint32_t* vals_out,
-                                 cudaStream_t stream);
+// Stable sort of (keys, vals) in place (dsmc_stage_sort): count (nkeys + 1
+// words), tile_sum and meta zeroed before the call; start gets the nkeys + 1
+// exclusive starts; scratch 2 n words.
+cudaError_t launch_sort(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t nkeys, uint32_t* count,
+                        uint32_t* start, uint32_t* tile_sum, uint32_t* scratch, Meta* meta, cudaStream_t stream);
+// NTC collisions of every cell of the sorted velocities p.in, in place
+// (collide stage).
+cudaError_t launch_collide_cells(const StepParams& p, cudaStream_t stream);
 cudaError_t launch_bounds_reorder(const uint32_t* keys, const uint32_t* idx, uint32_t n,
                                   uint32_t ncells, uint32_t* cse, const float* const src[6],
                                   float* const dst[6], cudaStream_t stream);

@@ -17,17 +17,17 @@ constexpr size_t kMaxTiles = (kMaxKeys + dsmcb::kScanTile - 1) / dsmcb::kScanTil
 static_assert(kMaxTiles <= (size_t)dsmcb::kMaxScanTiles, "key range beyond the scan tiles");
 
 // Fixed layout of the scratch: per-key counts and starts, scan-tile sums,
-// per-element tickets, scattered values and positions, the scan's counters.
-constexpr size_t kOffCount = 0;
+// scattered values and positions, the scan's counters.
+// The scan-tile sums and the counters lie before the counts, so that one
+// memset clears what a call needs cleared.
+constexpr size_t kOffTiles = 0;
+constexpr size_t kOffMeta = kOffTiles + align256(4 * kMaxTiles);
+constexpr size_t kOffCount = kOffMeta + align256(sizeof(dsmcb::Meta));
 constexpr size_t kOffStart = kOffCount + align256(4 * (kMaxKeys + 1));
-constexpr size_t kOffTiles = kOffStart + align256(4 * (kMaxKeys + 1));
-constexpr size_t kOffTicket = kOffTiles + align256(4 * kMaxTiles);
-constexpr size_t kOffVal = kOffTicket + align256(4 * kMaxN);
-constexpr size_t kOffPos = kOffVal + align256(4 * kMaxN);
-constexpr size_t kOffMeta = kOffPos + align256(4 * kMaxN);
-constexpr size_t kScratchBytes = kOffMeta + align256(sizeof(dsmcb::Meta));
+constexpr size_t kOffPairs = kOffStart + align256(4 * (kMaxKeys + 1));
+constexpr size_t kScratchBytes = kOffPairs + 2 * align256(4 * kMaxN);
 
-// About 13.6 MB of device memory, reserved on each device when the library's
+// About 9.4 MB of device memory, reserved on each device when the library's
 // kernels are loaded there.
 static __device__ __align__(256) unsigned char g_sort_scratch[kScratchBytes];
 
@@ -69,24 +69,14 @@ extern "C" int dsmc_stage_sort_static(uint32_t* keys, uint32_t* vals, uint32_t n
   cudaError_t e = scratch_address(&w);
   if (e != cudaSuccess) return DSMC_ERR_CUDA;
   cudaStream_t s = (cudaStream_t)stream;
-  const uint32_t tiles = (nkeys + dsmcb::kScanTile - 1) / dsmcb::kScanTile;
   uint32_t* count = reinterpret_cast<uint32_t*>(w + kOffCount);
-  uint32_t* start = reinterpret_cast<uint32_t*>(w + kOffStart);
+  uint32_t* start = cell_start ? cell_start : reinterpret_cast<uint32_t*>(w + kOffStart);
   uint32_t* tsum = reinterpret_cast<uint32_t*>(w + kOffTiles);
-  uint32_t* ticket = reinterpret_cast<uint32_t*>(w + kOffTicket);
-  uint32_t* tval = reinterpret_cast<uint32_t*>(w + kOffVal);
-  uint32_t* tpos = reinterpret_cast<uint32_t*>(w + kOffPos);
+  uint32_t* pairs = reinterpret_cast<uint32_t*>(w + kOffPairs);
   dsmcb::Meta* meta = reinterpret_cast<dsmcb::Meta*>(w + kOffMeta);
-  // counts, scan-tile sums and the scan's counters start every call at zero;
-  // the other regions are fully written before they are read
-  e = cudaMemsetAsync(count, 0, 4ull * (nkeys + 1), s);
-  if (!e) e = cudaMemsetAsync(tsum, 0, 4ull * tiles, s);
-  if (!e) e = cudaMemsetAsync(meta, 0, sizeof(dsmcb::Meta), s);
-  if (!e && n) e = dsmcb::launch_count_keys(keys, n, nkeys, ticket, count, tsum, tiles, s);
-  if (!e) e = dsmcb::launch_scan(count, nullptr, start, nkeys, tsum, tiles, meta, 0, s);
-  if (!e && n) e = dsmcb::launch_scatter_kv(keys, vals, ticket, start, n, nkeys, tval, tpos, s);
-  if (!e && n) e = dsmcb::launch_segment_fixup(start, nkeys, tval, tpos, keys, vals, s);
-  if (!e && cell_start)
-    e = cudaMemcpyAsync(cell_start, start, 4ull * (nkeys + 1), cudaMemcpyDeviceToDevice, s);
+  // scan-tile sums, the scan's counters and the counts start every call at
+  // zero; the other regions are fully written before they are read
+  e = cudaMemsetAsync(w, 0, kOffCount + 4ull * (nkeys + 1), s);
+  if (!e) e = dsmcb::launch_sort(keys, vals, n, nkeys, count, start, tsum, pairs, meta, s);
   return e ? DSMC_ERR_CUDA : DSMC_OK;
 }

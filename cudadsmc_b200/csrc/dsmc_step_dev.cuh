@@ -355,7 +355,8 @@ __device__ __forceinline__ void collide_cell(const StepParams& p, uint32_t cell,
 // two particles are not claimed by a lower lane, the others retry with the
 // same pair.  Acceptance uses (sigma*g)max as of the round's start.  M pairs
 // from vmax_in; returns the new (sigma*g)max (the same in every lane).
-// claim[] holds 0xffffffff for every claim index of the cell and is left so.
+// claim[] holds 0xffffffff for every claim index of the cell and is left so;
+// without one (null) the lanes compare their pairs with the lower lanes'.
 template <class Acc>
 __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint32_t cell,
                                                        uint32_t n, Acc acc, uint32_t* claim,
@@ -380,14 +381,23 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
     }
     drawn += want;
     uint32_t ji = 0, jj = 0;
-    if (pend) {
-      ji = acc.claim_index(pi);
-      jj = acc.claim_index(pj);
-      atomicMin(&claim[ji], lane);
-      atomicMin(&claim[jj], lane);
+    bool win = pend;
+    if (claim) {
+      if (pend) {
+        ji = acc.claim_index(pi);
+        jj = acc.claim_index(pj);
+        atomicMin(&claim[ji], lane);
+        atomicMin(&claim[jj], lane);
+      }
+      __syncwarp();
+      win = pend && claim[ji] == lane && claim[jj] == lane;
+    } else {
+      const unsigned pm = __ballot_sync(kFull, pend);
+      for (unsigned l = 0; l < 31; l++) {
+        const uint32_t li = __shfl_sync(kFull, pi, l), lj = __shfl_sync(kFull, pj, l);
+        if (l < lane && ((pm >> l) & 1u) && (li == pi || li == pj || lj == pi || lj == pj)) win = false;
+      }
     }
-    __syncwarp();
-    const bool win = pend && claim[ji] == lane && claim[jj] == lane;
     float vv = 0.f;
     if (win) {
       const float3 v1 = acc.get(pi), v2 = acc.get(pj);
@@ -404,7 +414,7 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
       }
     }
     __syncwarp();
-    if (pend) {
+    if (claim && pend) {
       claim[ji] = 0xffffffffu;
       claim[jj] = 0xffffffffu;
     }
@@ -786,13 +796,22 @@ template <class Acc>
 __device__ __forceinline__ void sample_cell(double* acc, uint32_t cells, uint32_t cell, int n,
                                             const Acc& a) {
   if (n <= 0) return;
+  // four particles' loads in flight, added one by one in order
   double su = 0, sv = 0, sw = 0, se = 0;
-  for (int k = 0; k < n; k++) {
-    const float3 q = a.get(k);
+  auto add = [&](float3 q) {
     const double x = q.x, y = q.y, z = q.z;
     su += x; sv += y; sw += z;
     se += x * x + y * y + z * z;
+  };
+  int k = 0;
+  for (; k + 4 <= n; k += 4) {
+    const float3 q0 = a.get(k), q1 = a.get(k + 1), q2 = a.get(k + 2), q3 = a.get(k + 3);
+    add(q0);
+    add(q1);
+    add(q2);
+    add(q3);
   }
+  for (; k < n; k++) add(a.get(k));
   acc[cell] += (double)n;
   acc[(size_t)cells + cell] += su;
   acc[2 * (size_t)cells + cell] += sv;

@@ -415,7 +415,7 @@ int dsmc_stage_sort(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t nkeys,
  * for callers that may not allocate device memory while they run, such as
  * code recording work into a memory-constrained pool or running next to a
  * caching allocator that owns the device.  The scratch is a fixed static
- * device array of about 13.6 MB, reserved on each device when the library's
+ * device array of about 9.4 MB, reserved on each device when the library's
  * kernels are loaded there; this call never calls cudaMalloc, cudaFree or an
  * allocating library function.
  * Limits: n <= DSMC_SORT_STATIC_MAX_N and nkeys <= DSMC_SORT_STATIC_MAX_KEYS;
