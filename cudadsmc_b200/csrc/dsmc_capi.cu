@@ -45,6 +45,7 @@ struct dsmc_handle {
   bool mt_on = false;
   double* acc = nullptr;
   double* cellbuf = nullptr;  // per-cell fields / sums, cell-major, for readback (on first use)
+  unsigned char* seedbuf = nullptr;  // scratch of the fill from fields (on first use)
   Meta* meta = nullptr;
   float* inj_rem = nullptr;
   uint32_t* inj_plan = nullptr;
@@ -189,7 +190,7 @@ void free_all(dsmc_handle* h) {
     h->A[i] = h->B[i] = nullptr;
   }
   void* ps[] = {h->orig, h->ntc_list, h->keys, h->cursor, h->count, h->start, h->tile_sum, h->maxrem, h->seeds,
-                h->acc, h->cellbuf, h->meta, h->inj_rem, h->inj_plan, h->gflags, h->gclear, h->greach, h->gslab,
+                h->acc, h->cellbuf, h->seedbuf, h->meta, h->inj_rem, h->inj_plan, h->gflags, h->gclear, h->greach, h->gslab,
                 h->gse, h->gtri, h->gplane, h->mt_state, h->mt_cfg};
   for (void* p : ps) cudaFree(p);
   h->mt_state = nullptr;
@@ -1087,20 +1088,14 @@ int outside_fractions(dsmc_handle* h, std::vector<float>& frac) {
   return DSMC_OK;
 }
 
-// Uploads the per-cell slots and counts, fills, resets the accumulators and
-// indexes the new state.
-int finish_fill(dsmc_handle* h, dsmcb::InitParams& ip, const std::vector<uint32_t>& slot,
-                const std::vector<uint32_t>& count, uint64_t n, uint32_t* n_out) {
-  if (n > h->capacity) return fail(h, DSMC_ERR_CAPACITY, "initial particles exceed capacity");
-  CK(h, cudaMemcpyAsync(h->start, slot.data(), (h->cells + 1) * 4, cudaMemcpyHostToDevice, h->stream),
-     "init upload");
-  CK(h, cudaMemcpyAsync(h->count, count.data(), (h->cells + 1) * 4, cudaMemcpyHostToDevice, h->stream),
-     "init upload");
+// Fills (the per-cell slots and counts of ip are on the device), resets the
+// accumulators and indexes the new state.
+int finish_fill(dsmc_handle* h, dsmcb::InitParams& ip, uint64_t n, uint32_t* n_out) {
   ip.grid = h->grid;
   ip.cells = h->cells;
-  ip.cell_slot = h->start;
-  ip.cell_count = h->count;
   ip.out = soa_of(h->A);
+  ip.redo = h->orig;  // dead between steps, as is the counter
+  ip.n_redo = &h->meta->n_defer;
   CK(h, dsmcb::launch_init_fill(ip, h->stream), "init fill");
   CK(h, cudaMemsetAsync(h->acc, 0, 5 * (size_t)h->cells * sizeof(double), h->stream), "reset samples");
   int st = reindex(h, (uint32_t)n);
@@ -1177,35 +1172,17 @@ int dsmc_init_state(dsmc_handle* h, const float stream_vel[3], uint32_t* n_out) 
   const float* sv = stream_vel ? stream_vel : c.stream_vel;
   ip.stream = make_float3(sv[0], sv[1], sv[2]);
   ip.seed = make_uint2((uint32_t)c.seed, (uint32_t)(c.seed >> 32));
-  return finish_fill(h, ip, slot, count, n, n_out);
+  if (n > h->capacity) return fail(h, DSMC_ERR_CAPACITY, "initial particles exceed capacity");
+  CK(h, cudaMemcpyAsync(h->start, slot.data(), (h->cells + 1) * 4, cudaMemcpyHostToDevice, h->stream),
+     "init upload");
+  CK(h, cudaMemcpyAsync(h->count, count.data(), (h->cells + 1) * 4, cudaMemcpyHostToDevice, h->stream),
+     "init upload");
+  ip.cell_slot = h->start;
+  ip.cell_count = h->count;
+  return finish_fill(h, ip, n, n_out);
 }
 
 namespace {
-
-// Free-stream share alpha of a cell with mean velocity u and temperature T
-// seen as a mixture of the free stream (U, T_inf) and a Maxwellian at the
-// wall temperature T_w with drift u_b: the mixture's mean and energy match
-// the cell's when
-//   alpha e_inf + (1 - alpha) e_w + |u - alpha U|^2 / (1 - alpha) = 3kT/m + |u|^2
-// (e = 3kT/m + |drift|^2 of a component), solved by bisection on
-// [0, 0.98]; 0 where the cell is colder than the wall or no root lies there.
-double two_stream_share(const double u[3], double T, const double U[3], double T_inf, double T_w,
-                        double kb_m) {
-  const double e_inf = 3.0 * kb_m * T_inf + U[0] * U[0] + U[1] * U[1] + U[2] * U[2];
-  const double e_w = 3.0 * kb_m * T_w;
-  const double rhs = 3.0 * kb_m * T + u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-  auto f = [&](double a) {
-    const double d0 = u[0] - a * U[0], d1 = u[1] - a * U[1], d2 = u[2] - a * U[2];
-    return a * e_inf + (1.0 - a) * e_w + (d0 * d0 + d1 * d1 + d2 * d2) / (1.0 - a) - rhs;
-  };
-  double lo = 0.0, hi = 0.98;
-  if (!(f(lo) < 0.0 && f(hi) > 0.0)) return 0.0;
-  for (int it = 0; it < 60; it++) {
-    const double mid = 0.5 * (lo + hi);
-    (f(mid) > 0.0 ? hi : lo) = mid;
-  }
-  return 0.5 * (lo + hi);
-}
 
 // dsmc_init_from_fields and its two-stream form (weight > 0).
 int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_t* n_out) {
@@ -1214,67 +1191,52 @@ int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_
   if (!(weight >= 0.f && weight <= 1.f)) return fail(h, DSMC_ERR_ARG, "two-stream weight outside [0, 1]");
   const bool two = weight > 0.f;
   if (two && !(c.wall_temp > 0.f)) return fail(h, DSMC_ERR_ARG, "two-stream fill needs a wall temperature");
-  std::vector<float> frac;
-  int st = outside_fractions(h, frac);
-  if (st) return st;
-  std::vector<uint32_t> slot(h->cells + 1), count(h->cells + 1, 0u);
-  std::vector<float4> state(h->cells);
-  std::vector<float2> maxrem(h->cells);
-  std::vector<float> share(two ? h->cells : 0);
-  const double U[3] = {c.stream_vel[0], c.stream_vel[1], c.stream_vel[2]};
   const bool geo = h->has_geom && c.geometry;
   const float kb_m = 1.3806e-23f / c.gas_mass;
-  uint64_t mix = c.seed ^ 0x2545F4914F6CDD1Dull;
-  uint64_t n = 0;
-  uint32_t kmax = 0;
-  for (uint32_t cell = 0; cell < h->cells; cell++) {
-    const float* f = fields5 + 5 * (size_t)cell;
-    // n is averaged over the whole cell volume (as dsmc_read_fields gives
-    // it), so a cell the body cuts receives its n V_c / F_N particles in the
-    // part outside the body; a cell the body covers stays empty
-    const double expect = (std::isfinite(f[0]) && f[0] > 0.f && frac[cell] > 0.f)
-                              ? (double)f[0] * h->cell_volume / c.fnum : 0.0;
-    const double fl = std::floor(expect);
-    const uint32_t k = (uint32_t)fl + (unit_draw(mix) < expect - fl ? 1u : 0u);
-    slot[cell] = (uint32_t)n;
-    count[cell] = k;
-    kmax = std::max(kmax, k);
-    n += k;
-    const float T = (std::isfinite(f[4]) && f[4] > 0.f) ? f[4] : c.temp;
-    state[cell] = make_float4(std::isfinite(f[1]) ? f[1] : 0.f, std::isfinite(f[2]) ? f[2] : 0.f,
-                              std::isfinite(f[3]) ? f[3] : 0.f, std::sqrt(kb_m * T));
-    if (two) {
-      // the share alpha from the free stream, the rest a Maxwellian whose
-      // drift and temperature keep the cell's mean and energy (the wall
-      // temperature itself at weight 1)
-      const double u[3] = {state[cell].x, state[cell].y, state[cell].z};
-      const double a = weight * two_stream_share(u, T, U, c.temp, c.wall_temp, kb_m);
-      share[cell] = (float)a;
-      if (a > 0.0) {
-        double ub[3], ub2 = 0.0, uu = 0.0, UU = 0.0;
-        for (int q = 0; q < 3; q++) {
-          ub[q] = (u[q] - a * U[q]) / (1.0 - a);
-          ub2 += ub[q] * ub[q];
-          uu += u[q] * u[q];
-          UU += U[q] * U[q];
-        }
-        const double e = (3.0 * kb_m * T + uu - a * (3.0 * kb_m * c.temp + UU)) / (1.0 - a) - ub2;
-        state[cell] = make_float4((float)ub[0], (float)ub[1], (float)ub[2],
-                                  (float)std::sqrt(std::max(e / 3.0, 0.0)));
-      }
-    }
-    // (sigma g)max scaled to the cell's temperature like the initial value
-    // (InitSimulationProperties, kernels/dsmc_kernel.cu:329-331)
-    maxrem[cell] = make_float2(h->max_rel_vel * std::sqrt(std::max(T, c.temp) / c.temp),
-                               (float)unit_draw(mix));
-  }
-  CK(h, cudaMemcpyAsync(fill_state(h), state.data(), h->cells * sizeof(float4), cudaMemcpyHostToDevice,
-                        h->stream), "seed upload");
-  CK(h, cudaMemcpyAsync(h->maxrem, maxrem.data(), h->cells * sizeof(float2), cudaMemcpyHostToDevice,
-                        h->stream), "seed upload");
-  if (two)
-    CK(h, cudaMemcpyAsync(fill_mix(h), share.data(), h->cells * sizeof(float), cudaMemcpyHostToDevice,
-                          h->stream), "seed upload");
+  // scratch of the handle: the fields, per-cell collision state, counts and
+  // slots, the scan's tile sums and counters, the totals
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t nc = h->cells;
+  const size_t o_mr = up(5 * nc * 4), o_slot = o_mr + up(8 * nc), o_count = o_slot + up(4 * (nc + 1));
+  const size_t o_tile = o_count + up(4 * (nc + 1)), o_meta = o_tile + up(4 * (size_t)h->n_scan_tiles);
+  const size_t o_tot = o_meta + up(sizeof(Meta)), bytes = o_tot + up(sizeof(dsmcb::SeedTotals));
+  if (!h->seedbuf) CK(h, dalloc(&h->seedbuf, bytes), "seed buffer alloc");
+  unsigned char* w = h->seedbuf;
+  if (geo)
+    CK(h, dsmcb::launch_outside_fraction(h->grid, base_params(h, c.dt).geom, h->cells, fill_frac(h), fill_point(h),
+                                         h->stream), "outside fraction");
+  CK(h, cudaMemcpyAsync(w, fields5, 5 * nc * sizeof(float), cudaMemcpyHostToDevice, h->stream), "seed upload");
+  CK(h, cudaMemsetAsync(w + o_count, 0, bytes - o_count, h->stream), "memset");
+  dsmcb::SeedParams sp{};
+  sp.fields = (const float*)w;
+  sp.cells = h->cells;
+  sp.frac = geo ? fill_frac(h) : nullptr;
+  sp.cell_volume = h->cell_volume;
+  sp.fnum = c.fnum;
+  sp.temp = c.temp;
+  sp.wall_temp = c.wall_temp;
+  sp.kb_m = kb_m;
+  sp.max_rel_vel = h->max_rel_vel;
+  sp.weight = weight;
+  for (int q = 0; q < 3; q++) sp.stream[q] = c.stream_vel[q];
+  sp.seed = c.seed ^ 0x2545F4914F6CDD1Dull;
+  sp.state = fill_state(h);
+  sp.share = two ? fill_mix(h) : nullptr;
+  sp.maxrem = (float2*)(w + o_mr);
+  sp.count = (uint32_t*)(w + o_count);
+  sp.tile_sum = (uint32_t*)(w + o_tile);
+  sp.totals = (dsmcb::SeedTotals*)(w + o_tot);
+  CK(h, dsmcb::launch_seed_cells(sp, h->stream), "seed cells");
+  CK(h, dsmcb::launch_scan(sp.count, nullptr, (uint32_t*)(w + o_slot), h->cells, sp.tile_sum, h->n_scan_tiles,
+                           (Meta*)(w + o_meta), 0, h->stream), "seed scan");
+  dsmcb::SeedTotals tot{};
+  CK(h, cudaMemcpyAsync(&tot, sp.totals, sizeof(tot), cudaMemcpyDeviceToHost, h->stream), "seed totals");
+  CK(h, cudaStreamSynchronize(h->stream), "seed totals");
+  const uint64_t n = tot.n;
+  const uint32_t kmax = tot.kmax;
+  if (n > h->capacity) return fail(h, DSMC_ERR_CAPACITY, "initial particles exceed capacity");
+  CK(h, cudaMemcpyAsync(h->maxrem, sp.maxrem, nc * sizeof(float2), cudaMemcpyDeviceToDevice, h->stream),
+     "seed collision state");
   dsmcb::InitParams ip{};
   ip.ppc = kmax;
   ip.kind = DSMC_INIT_MAXWELL;
@@ -1290,7 +1252,8 @@ int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_
     ip.geom = base_params(h, c.dt).geom;
     ip.cell_point = fill_point(h);
   }
-  return finish_fill(h, ip, slot, count, n, n_out);
+  ip.cell_slot = (const uint32_t*)(w + o_slot);
+  return finish_fill(h, ip, n, n_out);
 }
 
 }  // namespace

@@ -261,6 +261,27 @@ cudaError_t launch_sample_cells(const float* u, const float* v, const float* w,
                                 const uint32_t* start, uint32_t cells, double* acc,
                                 size_t fstride, size_t cstride, cudaStream_t stream);
 
+// Per-cell part of the fill from fields (dsmc_seed.cu).
+struct SeedTotals {
+  unsigned long long n;  // particles
+  uint32_t kmax;         // most in one cell
+};
+struct SeedParams {
+  const float* fields;   // per cell n, u, v, w, T
+  uint32_t cells;
+  const float* frac;     // fraction of the cell outside the body (null: all 1)
+  float cell_volume, fnum, temp, wall_temp, kb_m, max_rel_vel, weight;
+  float stream[3];
+  uint64_t seed;         // of the SplitMix64 draws, two per cell
+  float4* state;         // out: Maxwellian (u, v, w, sqrt(kT/m)), share drawn from the
+  float* share;          // free stream (null: none), (sigma g)max and remainder, count
+  float2* maxrem;
+  uint32_t* count;
+  uint32_t* tile_sum;    // added to: particles per scan tile, and the totals
+  SeedTotals* totals;
+};
+cudaError_t launch_seed_cells(const SeedParams& p, cudaStream_t stream);
+
 // Initial fill (dsmc_init_state).
 struct InitParams {
   GridGeom grid;
@@ -273,11 +294,13 @@ struct InitParams {
   float3 stream;
   uint2 seed;
   const uint32_t* cell_slot;  // per cell: first particle index, kNone = skipped cell
-  const uint32_t* cell_count; // per cell: particles to fill (<= ppc)
+  const uint32_t* cell_count; // per cell: particles to fill (<= ppc); null: up to the next slot
   const float4* cell_state;   // optional per cell (u, v, w, sqrt(kT/m)) of the Maxwellian
   const float* cell_mix;      // optional per cell (with cell_state): the fraction of particles
                               // drawn from the free stream (stream, vstd) instead
   int reject_inside;          // redraw positions that fall inside the mesh
+  uint32_t* redo;             // with reject_inside: the particles whose first position does,
+  uint32_t* n_redo;           // listed for the redraw kernel (room for all; the count zeroed)
   GeomView geom;
   const float4* cell_point;   // optional per cell: a point outside the mesh (w = 1) or none (w = 0)
   SoA out;
