@@ -82,6 +82,13 @@ class MoveParams(ctypes.Structure):
 _P = ctypes.c_void_p
 _U32 = ctypes.c_uint32
 _I = ctypes.c_int
+class Mlp(ctypes.Structure):
+    """dsmc_mlp"""
+    _fields_ = [(k, ctypes.c_int) for k in ("n_in", "in_pad", "hidden", "depth", "modes", "fields")] + [
+        ("w", ctypes.POINTER(_P)), ("b", ctypes.POINTER(_P)), ("w_out", _P), ("b_out", _P), ("basis", _P),
+        ("mean", _P)]
+
+
 SIGNATURES = [
     ("dsmc_config_default", _I, [ctypes.POINTER(Config)]),
     ("dsmc_config_read_xml", _I, [ctypes.c_char_p, ctypes.POINTER(Config)]),
@@ -129,6 +136,7 @@ SIGNATURES = [
     ("dsmc_gemm_split_workspace", ctypes.c_size_t, [_I, _I, _I]),
     ("dsmc_gemm_split_bf16", _I, [_I, _I, _I, _P, _I, _I, _P, _I, _I, _P, _P, _I, _P, _P]),
     ("dsmc_decode_mse", _I, [_I, _I, _I, _P, _P, _P, _P, ctypes.c_float, _P, _P, _P, _P, _P, _P]),
+    ("dsmc_mlp_forward", _I, [_P, _P, _I, _P, _P, _P, _P, _P, _P]),
     ("dsmc_gemm_check", _I, [_P]),
     ("dsmc_gelu_backward", _I, [_P, _P, _P, _P, ctypes.c_size_t, _P]),
     ("dsmc_colsum", _I, [_P, _I, _I, _I, _P, _P]),

@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 
 #include "dsmc_b200.h"
 #include "dsmc_kernels.cuh"
@@ -576,6 +577,23 @@ __global__ void __launch_bounds__(256) k_sum_splits(const float* __restrict__ pa
   }
 }
 
+// The network's inputs, handed over in the kernel's parameters (a copy from
+// pageable host memory would first wait for the stream): BF16, rows padded
+// with zeros to `pad`.
+template <int N>
+struct InputBlock {
+  float v[N];
+};
+template <int N>
+__global__ void __launch_bounds__(256) k_inputs(const __grid_constant__ InputBlock<N> x, int row0, int rows, int n_in,
+                                                int pad, bf16* out) {
+  chained_entry();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows * pad; i += gridDim.x * blockDim.x) {
+    const int r = i / pad, c = i - r * pad;
+    out[(size_t)(row0 + r) * pad + c] = __float2bfloat16(c < n_in ? x.v[r * n_in + c] : 0.f);
+  }
+}
+
 // ------------------------------------------------------------------- host ----
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -677,6 +695,14 @@ int run(GemmArgs g, const void* a, int lda, int a_trans, const void* b, int ldb,
   return e == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
 }
 
+template <int N>
+cudaError_t launch_inputs(const float* x, int row0, int rows, int n_in, int pad, bf16* out, cudaStream_t s) {
+  InputBlock<N> b;
+  std::memcpy(b.v, x + (size_t)row0 * n_in, (size_t)rows * n_in * sizeof(float));
+  return launch_chained(k_inputs<N>, grid_for((uint64_t)rows * pad, 256, 1), 256, 0, s, true, b, row0, rows, n_in, pad,
+                        out);
+}
+
 }  // namespace
 
 extern "C" {
@@ -747,6 +773,39 @@ int dsmc_decode_mse(int m, int n, int k, const void* a, const void* b, const flo
   g.loss = loss;
   g.count = count;
   return run<true>(g, a, k, 0, b, n, 0, (cudaStream_t)stream);
+}
+
+int dsmc_mlp_forward(const dsmc_mlp* n, const float* x, int batch, void* xb, float* const* z, void* const* h, void* cb,
+                     float* y, void* stream) {
+  if (!n || !x || batch <= 0 || !xb || !h || !cb || n->depth < 0 || n->n_in <= 0 ||
+      n->in_pad < n->n_in || n->n_in > 4096)
+    return DSMC_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  // as many rows per launch as the parameters hold
+  const int small = 1000, large = 4096;
+  for (int r = 0; r < batch;) {
+    const bool few = (batch - r) * (int64_t)n->n_in <= small;
+    const int rows = std::min(batch - r, (few ? small : large) / n->n_in);
+    const cudaError_t e = few ? launch_inputs<small>(x, r, rows, n->n_in, n->in_pad, static_cast<bf16*>(xb), s)
+                              : launch_inputs<large>(x, r, rows, n->n_in, n->in_pad, static_cast<bf16*>(xb), s);
+    if (e != cudaSuccess) return DSMC_ERR_CUDA;
+    r += rows;
+  }
+  const void* in = xb;
+  int k = n->in_pad;
+  for (int l = 0; l < n->depth; l++) {
+    const int st = dsmc_gemm_bf16(batch, n->hidden, k, in, k, 0, n->w[l], n->hidden, 0, z ? z[l] : nullptr, n->hidden,
+                                  0.f, n->b[l], 1, h[l], n->hidden, 1, stream);
+    if (st != DSMC_OK) return st;
+    in = h[l];
+    k = n->hidden;
+  }
+  int st = dsmc_gemm_bf16(batch, n->modes, k, in, k, 0, n->w_out, n->modes, 0, nullptr, 0, 0.f, n->b_out, 0, cb,
+                          n->modes, 1, stream);
+  if (st == DSMC_OK && y)
+    st = dsmc_gemm_bf16(batch, n->fields, n->modes, cb, n->modes, 0, n->basis, n->fields, 0, y, n->fields, 0.f,
+                        n->mean, 0, nullptr, 0, 1, stream);
+  return st;
 }
 
 int dsmc_gemm_check(void* stream) {

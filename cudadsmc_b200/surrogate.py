@@ -15,7 +15,7 @@ import math
 
 import numpy as np
 
-from ._capi import check, lib
+from ._capi import Mlp, check, lib
 
 _P = ctypes.c_void_p
 
@@ -75,48 +75,48 @@ class WarmStartMLP:
         """Sets the field mean (the decoder bias), e.g. the training-set mean."""
         self.params["mean"].copy_(self.torch.as_tensor(mean, dtype=self.torch.float32))
 
-    def _inputs(self, x):
-        torch = self.torch
-        xb = np.zeros((len(x), self.IN_PAD), np.float32)
-        xb[:, : self.n_in] = x
-        xf = torch.from_numpy(xb).to(self.dev)
-        out = torch.empty(xf.shape, dtype=torch.bfloat16, device=self.dev)
-        check(lib().dsmc_to_bf16(_p(xf), _p(out), xf.numel(), _stream()), "to_bf16")
-        return out
-
     # ------------------------------------------------------------ forward --
-    def _coefficients(self, x):
-        """The hidden layers and the coefficients: the cache for backward."""
+    def _forward(self, x, cache, field):
+        """One call for the whole pass: padded inputs, layers, coefficients and,
+        with `field`, the field.  Returns (field or None, cache for backward or
+        None): the cache holds every layer's input and pre-activation."""
         torch = self.torch
-        B = len(x)
-        h = self._inputs(x)
-        cache = {"x": [], "z": []}
-        for l in range(self.depth):
-            W = self.bf[f"W{l}"]
-            z = torch.empty((B, self.hidden), dtype=torch.float32, device=self.dev)
-            hn = torch.empty((B, self.hidden), dtype=torch.bfloat16, device=self.dev)
-            self._gemm(B, self.hidden, W.shape[0], h, h.shape[1], 0, W, self.hidden, 0, z, self.hidden,
-                       bias=self.params[f"b{l}"], act=1, cb=hn, ldcb=self.hidden)
-            cache["x"].append(h)
-            cache["z"].append(z)
-            h = hn
-        cache["h"] = h
-        c = torch.empty((B, self.modes), dtype=torch.float32, device=self.dev)
-        cb = torch.empty((B, self.modes), dtype=torch.bfloat16, device=self.dev)
-        self._gemm(B, self.modes, self.hidden, h, self.hidden, 0, self.bf["Wout"], self.modes, 0, c,
-                   self.modes, bias=self.params["bout"], cb=cb, ldcb=self.modes)
-        cache["c"] = cb
-        return cache
+        B, H, D = len(x), self.hidden, self.depth
+        xin = np.empty((B, self.n_in), np.float32)
+        xin[:] = x
+        ptrs = _P * max(D, 1)
+        net = Mlp(self.n_in, self.IN_PAD, H, D, self.modes, self.F)
+        net.w = ptrs(*[self.bf[f"W{l}"].data_ptr() for l in range(D)])
+        net.b = ptrs(*[self.params[f"b{l}"].data_ptr() for l in range(D)])
+        net.w_out, net.b_out = self.bf["Wout"].data_ptr(), self.params["bout"].data_ptr()
+        net.basis, net.mean = self.bf["B"].data_ptr(), self.params["mean"].data_ptr()
+        # 16-bit activations in one buffer (256-byte rows apart), 32-bit
+        # pre-activations only where backward will ask for them
+        parts = [B * self.IN_PAD] + [B * H] * D + [B * self.modes]
+        offs = [0]
+        for n in parts:
+            offs.append(offs[-1] + (n + 127) // 128 * 128)
+        act = torch.empty(offs[-1], dtype=torch.bfloat16, device=self.dev)
+        base = act.data_ptr()
+        ptr = [base + 2 * o for o in offs]
+        h = ptrs(*ptr[1:D + 1])
+        zp = z = None
+        if cache:
+            z = torch.empty((max(D, 1), B, H), dtype=torch.float32, device=self.dev)
+            zp = ptrs(*[z.data_ptr() + 4 * B * H * l for l in range(D)])
+        y = torch.empty((B, self.F), dtype=torch.float32, device=self.dev) if field else None
+        check(lib().dsmc_mlp_forward(ctypes.byref(net), xin.ctypes.data, B, ptr[0], zp, h, ptr[D + 1], _p(y), _stream()),
+              "mlp_forward")
+        if not cache:
+            return y, None
+        rows = [self.IN_PAD] + [H] * D + [self.modes]
+        a = [act[o:o + n].view(B, c) for o, n, c in zip(offs, parts, rows)]
+        return y, {"x": a[:D], "z": [z[l] for l in range(D)], "h": a[D], "c": a[D + 1]}
 
     def forward(self, x):
         """x: [batch, n_in] normalized inputs.  Returns the field [batch, F]
         (FP32, on the device) and the cache for backward."""
-        B = len(x)
-        cache = self._coefficients(x)
-        y = self.torch.empty((B, self.F), dtype=self.torch.float32, device=self.dev)
-        self._gemm(B, self.F, self.modes, cache["c"], self.modes, 0, self.bf["B"], self.F, 0, y, self.F,
-                   bias=self.params["mean"])
-        return y, cache
+        return self._forward(x, cache=True, field=True)
 
     # ----------------------------------------------------------- backward --
     def loss_and_grads(self, x, targets_bf16):
@@ -124,7 +124,7 @@ class WarmStartMLP:
         Returns (loss, valid count, grads dict of FP32 tensors)."""
         torch = self.torch
         B = len(x)
-        cache = self._coefficients(x)
+        _, cache = self._forward(x, cache=True, field=False)
         y = torch.empty((B, self.F), dtype=torch.float32, device=self.dev)
         n = B * self.F
         dyb = torch.empty(y.shape, dtype=torch.bfloat16, device=self.dev)
@@ -207,5 +207,4 @@ class WarmStartMLP:
         return history
 
     def predict(self, x):
-        y, _ = self.forward(np.asarray(x, np.float32))
-        return y
+        return self._forward(x, cache=False, field=True)[0]

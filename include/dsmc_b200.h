@@ -550,6 +550,24 @@ int dsmc_gemm_split_bf16(int m, int n, int k, const void* a, int lda, int a_tran
 int dsmc_decode_mse(int m, int n, int k, const void* a, const void* b, const float* bias, const void* t_bf16,
                     float scale, float* y, void* dy_bf16, float* dy_colsum, double* loss,
                     unsigned long long* count, void* stream);
+/* The network's forward pass in one call: `batch` rows of n_in inputs in host
+ * memory (taken before the call returns), padded to in_pad columns; depth
+ * layers of `hidden` GELU units; `modes` coefficients; the field, unless y is
+ * NULL.  Weights in BF16 (in_pad or hidden x hidden, hidden x modes, modes x
+ * fields), biases in FP32.  xb receives the padded inputs, h[l] the
+ * activations and cb the coefficients in BF16, z[l] (z may be NULL) the
+ * pre-activations in FP32; device pointers, rows without padding. */
+typedef struct dsmc_mlp {
+  int n_in, in_pad, hidden, depth, modes, fields;
+  const void* const* w; /* depth weights and biases */
+  const float* const* b;
+  const void* w_out;
+  const float* b_out;
+  const void* basis;
+  const float* mean;
+} dsmc_mlp;
+int dsmc_mlp_forward(const dsmc_mlp* net, const float* x, int batch, void* xb, float* const* z, void* const* h,
+                     void* cb, float* y, void* stream);
 /* Synchronises `stream` and reports whether a dsmc_gemm_bf16 launch since
  * the last check gave up waiting on its tensor-core work (DSMC_ERR_DEVICE;
  * its output is then incomplete); clears the flag. */
