@@ -54,6 +54,8 @@ struct GemmArgs {
   int ldcb;
   int tma_t;          // the targets come by TMA
   int tma_c, tma_cb;  // the output goes out by TMA (its rows 16-byte aligned)
+  int b_early;        // B is not written by the kernel before this one: its first tiles may be
+                      // fetched while that one finishes
   int part_rows;      // > 0: split z writes its own m x n product, part_rows rows further down per split
   // the fused error (MSE kernels): targets, scale, column sums, loss, count
   const bf16* t;
@@ -66,8 +68,9 @@ struct GemmArgs {
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678f)); }
 
-// Epilogue warps: four (one per quarter of the accumulator's lanes); for the
-// error sixteen, four per quarter taking every fourth block of 32 columns.
+// Epilogue warps: four (one per quarter of the accumulator's lanes); one per
+// 32 x 32 block of the tile where the tile is narrow (a layer's GELU, one tile
+// per CTA, is then half as long), and for the error: sixteen, four per quarter taking every fourth block of 32 columns.
 // Its 900 instructions per block are chains of short waits (accumulator,
 // targets, FP64 sum, column sum), so its time falls with the warps that share
 // a scheduler: 1024 x 327680 x 256 took 1026 us with four, 890 with eight, 610 with
@@ -77,9 +80,10 @@ __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z
 template <int BN, bool MSE>
 struct Shape {
   static constexpr int kStages = BN == 256 || MSE ? 3 : BN == 128 ? 4 : 6;
-  static constexpr int kEpiWarps = MSE ? BN / 8 : 4;  // MSE: one per block of the tile
+  static constexpr int kEpiWarps = MSE || BN == 64 ? BN / 8 : 4;  // BN / 8: one per block of the tile
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
-  static constexpr int kStaging = MSE ? 1 : 2;
+  static constexpr bool kOneBlock = kEpiWarps == BN / 8;
+  static constexpr int kStaging = kOneBlock ? 1 : 2;
   static constexpr int kABytes = umma::kBM * umma::kBK * 2;
   static constexpr int kBBytes = BN * umma::kBK * 2;
   static constexpr uint32_t kTmemCols = 2 * BN;
@@ -110,7 +114,7 @@ struct __align__(128) Smem {
   unsigned char f[Sh::kEpiWarps][Sh::kStaging][4096];
   unsigned char h[Sh::kEpiWarps][Sh::kStaging][2048];
   MseSmem<BN, MSE> mse;
-  alignas(16) float bias[Sh::kEpiWarps][MSE ? 32 : BN];
+  alignas(16) float bias[Sh::kEpiWarps][Sh::kOneBlock ? 32 : BN];
   unsigned long long full[Sh::kStages], empty[Sh::kStages];
   unsigned long long tfull[2], tempty[2], drain;
   uint32_t tmem_base;
@@ -250,6 +254,26 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
   fence_after_sync();
   const uint32_t tmem = sm.tmem_base;
   volatile uint32_t* failed = &sm.failed;
+  auto load_b = [&](int s, int nt, int kx) {
+    if (g.b_mn) {
+#pragma unroll
+      for (int q = 0; q < BN / 64; q++)
+        tma_load(sm.b[s] + 8192 * q, &map_b, nt * BN + 64 * q, kx, &sm.full[s]);
+    } else {
+      tma_load(sm.b[s], &map_b, kx, nt * BN, &sm.full[s]);
+    }
+  };
+  int early = 0;  // stages whose B is on its way already
+  if (g.b_early && warp == 0 && lane == 0) {
+    int mt, nt, z;
+    if (TileWalk(g, MSE).get(mt, nt, z)) {
+      early = min(S, k_tiles(g, z));
+      for (int j = 0; j < early; j++) {
+        mbar_expect_tx(&sm.full[j], Sh::kABytes + Sh::kBBytes);
+        load_b(j, nt, z * g.kchunk + j * kBK);
+      }
+    }
+  }
   // everything above ran beside the kernel before this one
   chained_entry();
 
@@ -267,20 +291,16 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
           ok = false;
           break;
         }
-        mbar_expect_tx(&sm.full[s], Sh::kABytes + Sh::kBBytes);
         const int kx = k0 + j * kBK;
+        if (it >= early) {
+          mbar_expect_tx(&sm.full[s], Sh::kABytes + Sh::kBBytes);
+          load_b(s, nt, kx);
+        }
         if (g.a_mn) {
           tma_load(sm.a[s], &map_a, mt * kBM, kx, &sm.full[s]);
           tma_load(sm.a[s] + 8192, &map_a, mt * kBM + 64, kx, &sm.full[s]);
         } else {
           tma_load(sm.a[s], &map_a, kx, mt * kBM, &sm.full[s]);
-        }
-        if (g.b_mn) {
-#pragma unroll
-          for (int q = 0; q < BN / 64; q++)
-            tma_load(sm.b[s] + 8192 * q, &map_b, nt * BN + 64 * q, kx, &sm.full[s]);
-        } else {
-          tma_load(sm.b[s], &map_b, kx, nt * BN, &sm.full[s]);
         }
       }
     }
@@ -341,14 +361,14 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
       if (g.tma_t && lane == 0) targets.issue(g, &map_t, sm.mse, ew, quad, ew >> 2);
     }
     // the bias of a tile's columns, asked for one tile ahead
-    constexpr int kBlocks = MSE ? 1 : BN / 32;  // per warp and tile
+    constexpr int kBlocks = Sh::kOneBlock ? 1 : BN / 32;  // per warp and tile
     float bv[kBlocks];
     auto load_bias = [&](const TileWalk& w) {
       int mt, nt, z;
       const bool there = w.get(mt, nt, z);
 #pragma unroll
       for (int q = 0; q < kBlocks; q++) {
-        const int c = nt * BN + 32 * (MSE ? ew >> 2 : q) + lane;
+        const int c = nt * BN + 32 * (Sh::kOneBlock ? ew >> 2 : q) + lane;
         bv[q] = there && c < g.n ? __ldg(g.bias + c) : 0.f;
       }
     };
@@ -373,12 +393,12 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
       const int row0 = mt * kBM + 32 * quad, row = row0 + lane;
       const uint32_t t0 = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(acc * BN);
 #pragma unroll 1
-      for (int q = MSE ? ew >> 2 : 0; q < BN / 32; q += MSE ? BN / 32 : 1) {
+      for (int q = Sh::kOneBlock ? ew >> 2 : 0; q < BN / 32; q += Sh::kOneBlock ? BN / 32 : 1) {
         const int c0 = nt * BN + 32 * q;
         const bool any = row0 < g.m && c0 < g.n;  // the warp's block has elements
         float v[32];
         ld32(t0 + (uint32_t)(32 * q), v);
-        if (MSE || q == BN / 32 - 1) {  // the accumulator is read: the next tile but one may overwrite it
+        if (Sh::kOneBlock || q == BN / 32 - 1) {  // the accumulator is read: the next tile but one may overwrite it
           fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&sm.tempty[acc]);
@@ -392,7 +412,7 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
         if (g.bias) {
 #pragma unroll
           for (int i = 0; i < 8; i++) {
-            const float4 b = *reinterpret_cast<const float4*>(sbias + (MSE ? 0 : 32 * q) + 4 * i);
+            const float4 b = *reinterpret_cast<const float4*>(sbias + (Sh::kOneBlock ? 0 : 32 * q) + 4 * i);
             v[4 * i] += b.x; v[4 * i + 1] += b.y; v[4 * i + 2] += b.z; v[4 * i + 3] += b.w;
           }
         }
@@ -707,9 +727,9 @@ cudaError_t launch_inputs(const float* x, int row0, int rows, int n_in, int pad,
 
 extern "C" {
 
-int dsmc_gemm_bf16(int m, int n, int k, const void* a, int lda, int a_trans, const void* b, int ldb,
-                   int b_trans, float* c, int ldc, float beta, const float* bias, int act, void* c_bf16,
-                   int ldcb, int split_k, void* stream) {
+static int gemm(int m, int n, int k, const void* a, int lda, int a_trans, const void* b, int ldb, int b_trans,
+                float* c, int ldc, float beta, const float* bias, int act, void* c_bf16, int ldcb, int split_k,
+                bool b_early, void* stream) {
   if (m <= 0 || n <= 0 || k <= 0 || !a || !b || (!c && !c_bf16)) return DSMC_ERR_ARG;
   // 16-byte rows along the contiguous dimension of each operand
   if (k % 8 || lda % 8 || ldb % 8 || !aligned16(a) || !aligned16(b)) return DSMC_ERR_ARG;
@@ -725,7 +745,14 @@ int dsmc_gemm_bf16(int m, int n, int k, const void* a, int lda, int a_trans, con
   const int per = (ksteps + split_k - 1) / split_k;
   g.kchunk = per * umma::kBK;
   g.splits = (k + g.kchunk - 1) / g.kchunk;
+  g.b_early = b_early;
   return run<false>(g, a, lda, a_trans != 0, b, ldb, b_trans != 0, (cudaStream_t)stream);
+}
+
+int dsmc_gemm_bf16(int m, int n, int k, const void* a, int lda, int a_trans, const void* b, int ldb,
+                   int b_trans, float* c, int ldc, float beta, const float* bias, int act, void* c_bf16,
+                   int ldcb, int split_k, void* stream) {
+  return gemm(m, n, k, a, lda, a_trans, b, ldb, b_trans, c, ldc, beta, bias, act, c_bf16, ldcb, split_k, false, stream);
 }
 
 int dsmc_gemm_split_bf16(int m, int n, int k, const void* a, int lda, int a_trans, const void* b, int ldb,
@@ -791,20 +818,22 @@ int dsmc_mlp_forward(const dsmc_mlp* n, const float* x, int batch, void* xb, flo
     if (e != cudaSuccess) return DSMC_ERR_CUDA;
     r += rows;
   }
+  // the weights are nothing that the kernels of this pass write, and whatever
+  // wrote them before the pass was complete before its first kernel's work
   const void* in = xb;
   int k = n->in_pad;
   for (int l = 0; l < n->depth; l++) {
-    const int st = dsmc_gemm_bf16(batch, n->hidden, k, in, k, 0, n->w[l], n->hidden, 0, z ? z[l] : nullptr, n->hidden,
-                                  0.f, n->b[l], 1, h[l], n->hidden, 1, stream);
+    const int st = gemm(batch, n->hidden, k, in, k, 0, n->w[l], n->hidden, 0, z ? z[l] : nullptr, n->hidden, 0.f,
+                        n->b[l], 1, h[l], n->hidden, 1, true, stream);
     if (st != DSMC_OK) return st;
     in = h[l];
     k = n->hidden;
   }
-  int st = dsmc_gemm_bf16(batch, n->modes, k, in, k, 0, n->w_out, n->modes, 0, nullptr, 0, 0.f, n->b_out, 0, cb,
-                          n->modes, 1, stream);
+  int st = gemm(batch, n->modes, k, in, k, 0, n->w_out, n->modes, 0, nullptr, 0, 0.f, n->b_out, 0, cb, n->modes, 1,
+                true, stream);
   if (st == DSMC_OK && y)
-    st = dsmc_gemm_bf16(batch, n->fields, n->modes, cb, n->modes, 0, n->basis, n->fields, 0, y, n->fields, 0.f,
-                        n->mean, 0, nullptr, 0, 1, stream);
+    st = gemm(batch, n->fields, n->modes, cb, n->modes, 0, n->basis, n->fields, 0, y, n->fields, 0.f, n->mean, 0,
+              nullptr, 0, 1, true, stream);
   return st;
 }
 
