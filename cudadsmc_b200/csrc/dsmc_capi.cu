@@ -222,6 +222,15 @@ void set_vhs_fast(dsmcb::StepParams& p, float cross_section, float omega, float 
   p.vhs_k = (float)((double)cross_section * std::pow((double)gref, e));
 }
 
+// One shared-memory share for a step's kernels (Chain) where the order kernel's
+// tiles fit one wave of 16 warps per SM, which that share holds; the driver's
+// choice elsewhere.
+int step_carveout(const dsmc_handle* h) {
+  return dsmcb::cell_kernel_is_warp(h->variant) && dsmcb::cell_kernel_chunk_capacity(h->variant) == 128 &&
+                 h->n_tiles <= 16u * (uint32_t)dsmcb::num_sms()
+             ? 65 : -1;
+}
+
 dsmcb::StepParams base_params(dsmc_handle* h, float dt) {
   dsmcb::StepParams p{};
   p.grid = h->grid;
@@ -276,6 +285,7 @@ dsmcb::StepParams base_params(dsmc_handle* h, float dt) {
   p.sample_every = h->cfg.sample_every;
   p.cells_per_tile = (int)h->cells_per_tile;
   p.n_tiles = h->n_tiles;
+  p.carveout = step_carveout(h);
   p.step_override = 0;
   return p;
 }
@@ -357,8 +367,8 @@ cudaError_t enqueue_inflow(dsmc_handle* h, float dt, uint2 seed, cudaStream_t st
   for (const auto& in : h->inflows) {
     const dsmcb::InjectParams ip = inject_params(h, in, dt, seed);
     const cudaError_t e = stream == h->stream
-                              ? timed(h, 3, [&] { return dsmcb::launch_inject(ip, stream); })
-                              : dsmcb::launch_inject(ip, stream);
+                              ? timed(h, 3, [&] { return dsmcb::launch_inject(ip, stream, step_carveout(h)); })
+                              : dsmcb::launch_inject(ip, stream, step_carveout(h));
     if (e) return e;
   }
   return cudaSuccess;
@@ -392,7 +402,7 @@ cudaError_t enqueue_step(dsmc_handle* h, float dt) {
   cudaError_t e;
   e = timed(h, 0, [&] {
     return dsmcb::launch_scan(h->count, h->cursor, h->start, h->cells, h->tile_sum,
-                              h->n_scan_tiles, h->meta, 1, h->stream);
+                              h->n_scan_tiles, h->meta, 1, h->stream, step_carveout(h));
   });
   if (e) return e;
   // the split cell kernels gather the state through orig themselves; the
@@ -401,7 +411,7 @@ cudaError_t enqueue_step(dsmc_handle* h, float dt) {
   e = timed(h, 1, [&] {
     return dsmcb::launch_scatter(!split, soa_of(h->A), soa_of(h->B), h->keys, h->start, h->cursor,
                                  h->orig, h->cells, h->tile_sum, h->n_scan_tiles, h->meta,
-                                 h->capacity, h->stream);
+                                 h->capacity, h->stream, step_carveout(h));
   });
   if (e) return e;
   dsmcb::StepParams p = step_params(h, dt, split);

@@ -1196,7 +1196,7 @@ cudaError_t launch_order_w(const StepParams& p, cudaStream_t stream) {
   const uint32_t need = (p.n_tiles + WARPS - 1) / WARPS;
   if (grid > need) grid = need;
   if (grid == 0) return cudaSuccess;
-  return launch_chained(k_order_w<CAPW, WARPS, MINB>, grid, WARPS * 32, smem, stream, true, p);
+  return launch_chained(k_order_w<CAPW, WARPS, MINB>, grid, WARPS * 32, smem, stream, Chain(true, p.carveout), p);
 }
 
 constexpr int kFlightWarps = 8;
@@ -1219,7 +1219,7 @@ cudaError_t launch_flight_w(const StepParams& p, cudaStream_t stream) {
   }
   // a full wave of warps: the particle count is known only on the device
   return launch_chained(k_flight_w<kFlightWarps, MINB>, (uint32_t)(num_sms() * ls.per_sm), kFlightWarps * 32,
-                        p.n_scan_tiles * 4u, stream, true, p);
+                        p.n_scan_tiles * 4u, stream, Chain(true, p.carveout), p);
 }
 
 template <int MINB>
@@ -1239,7 +1239,7 @@ cudaError_t launch_flight_pw(const StepParams& p, cudaStream_t stream) {
     ls.per_sm = per_sm;
   }
   return launch_chained(k_flight_pw<kFlightWarps, MINB>, (uint32_t)(num_sms() * ls.per_sm), kFlightWarps * 32,
-                        p.n_scan_tiles * 4u, stream, true, p);
+                        p.n_scan_tiles * 4u, stream, Chain(true, p.carveout), p);
 }
 
 constexpr int kNtcWarps = 8;
@@ -1259,7 +1259,7 @@ cudaError_t launch_ntc_w(const StepParams& p, cudaStream_t stream) {
     ls.device = dev;
     ls.per_sm = per_sm;
   }
-  return launch_chained(k_ntc_w<kNtcWarps>, (uint32_t)(num_sms() * ls.per_sm), kNtcWarps * 32, 0, stream, true, p);
+  return launch_chained(k_ntc_w<kNtcWarps>, (uint32_t)(num_sms() * ls.per_sm), kNtcWarps * 32, 0, stream, Chain(true, p.carveout), p);
 }
 
 template <int MINB, bool COOP>
@@ -1277,11 +1277,11 @@ cudaError_t launch_mesh_w(const StepParams& p, cudaStream_t stream) {
     ls.device = dev;
     ls.per_sm = per_sm;
   }
-  return launch_chained(k_mesh_w<MINB, COOP>, (uint32_t)(num_sms() * ls.per_sm), 32 * kMeshWarps, 0, stream, true, p);
+  return launch_chained(k_mesh_w<MINB, COOP>, (uint32_t)(num_sms() * ls.per_sm), 32 * kMeshWarps, 0, stream, Chain(true, p.carveout), p);
 }
 
 cudaError_t launch_sample_w(const StepParams& p, cudaStream_t stream) {
-  return launch_chained(k_sample_w, grid_for(p.cells, 256, 8), 256, 0, stream, true, p);
+  return launch_chained(k_sample_w, grid_for(p.cells, 256, 8), 256, 0, stream, Chain(true, p.carveout), p);
 }
 
 }  // namespace

@@ -901,8 +901,8 @@ cudaError_t launch_index(const GridGeom& g, uint32_t cells, const float* x, cons
 
 cudaError_t launch_scan(uint32_t* count, uint32_t* cursor, uint32_t* start, uint32_t cells,
                         const uint32_t* tile_sum, uint32_t n_scan_tiles, Meta* meta, int bump_step,
-                        cudaStream_t stream) {
-  return launch_chained(k_scan, n_scan_tiles, 256, 0, stream, true, count, cursor, start, cells, tile_sum, meta,
+                        cudaStream_t stream, int carveout) {
+  return launch_chained(k_scan, n_scan_tiles, 256, 0, stream, Chain(true, carveout), count, cursor, start, cells, tile_sum, meta,
                         bump_step);
 }
 
@@ -910,9 +910,9 @@ cudaError_t launch_scatter(bool with_state, const SoA& src, SoA dst, const uint3
                            const uint32_t* start,
                            uint32_t* cursor, uint32_t* orig, uint32_t cells, uint32_t* tile_sum,
                            uint32_t n_scan_tiles, Meta* meta, uint32_t capacity,
-                           cudaStream_t stream) {
+                           cudaStream_t stream, int carveout) {
   const uint32_t grid = (uint32_t)num_sms() * 4;
-  return launch_chained(with_state ? k_scatter<true> : k_scatter<false>, grid, 256, 0, stream, true, src, dst, keys,
+  return launch_chained(with_state ? k_scatter<true> : k_scatter<false>, grid, 256, 0, stream, Chain(true, carveout), src, dst, keys,
                         start, cursor, orig, cells, tile_sum, n_scan_tiles, meta, capacity);
 }
 
@@ -1366,10 +1366,10 @@ cudaError_t launch_inject_b(const BatchOf<InjectParams>& plan, uint32_t plan_blo
   return e;
 }
 
-cudaError_t launch_inject(const InjectParams& p, cudaStream_t stream) {
-  cudaError_t e = launch_chained(k_inject_plan, 1, 32, 0, stream, true, p, p.plan);
+cudaError_t launch_inject(const InjectParams& p, cudaStream_t stream, int carveout) {
+  cudaError_t e = launch_chained(k_inject_plan, 1, 32, 0, stream, Chain(true, carveout), p, p.plan);
   const uint32_t grid = (uint32_t)num_sms();
-  if (!e) e = launch_chained(k_inject_fill, grid, 256, p.n_scan_tiles * 4, stream, true, p, p.plan);
+  if (!e) e = launch_chained(k_inject_fill, grid, 256, p.n_scan_tiles * 4, stream, Chain(true, carveout), p, p.plan);
   return e;
 }
 
