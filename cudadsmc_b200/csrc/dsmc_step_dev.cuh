@@ -796,27 +796,30 @@ template <class Acc>
 __device__ __forceinline__ void sample_cell(double* acc, uint32_t cells, uint32_t cell, int n,
                                             const Acc& a) {
   if (n <= 0) return;
-  // four particles' loads in flight, added one by one in order
+  // the sums so far and up to eight particles' loads in flight together, the
+  // particles added one by one in order
+  double sum[5];
+#pragma unroll
+  for (int f = 0; f < 5; f++) sum[f] = acc[f * (size_t)cells + cell];
   double su = 0, sv = 0, sw = 0, se = 0;
-  auto add = [&](float3 q) {
-    const double x = q.x, y = q.y, z = q.z;
-    su += x; sv += y; sw += z;
-    se += x * x + y * y + z * z;
-  };
-  int k = 0;
-  for (; k + 4 <= n; k += 4) {
-    const float3 q0 = a.get(k), q1 = a.get(k + 1), q2 = a.get(k + 2), q3 = a.get(k + 3);
-    add(q0);
-    add(q1);
-    add(q2);
-    add(q3);
+  for (int k = 0; k < n; k += 8) {
+    float3 q[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (k + j < n) q[j] = a.get(k + j);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (k + j >= n) break;
+      const double x = q[j].x, y = q[j].y, z = q[j].z;
+      su += x; sv += y; sw += z;
+      se += x * x + y * y + z * z;
+    }
   }
-  for (; k < n; k++) add(a.get(k));
-  acc[cell] += (double)n;
-  acc[(size_t)cells + cell] += su;
-  acc[2 * (size_t)cells + cell] += sv;
-  acc[3 * (size_t)cells + cell] += sw;
-  acc[4 * (size_t)cells + cell] += se;
+  acc[cell] = sum[0] + (double)n;
+  acc[(size_t)cells + cell] = sum[1] + su;
+  acc[2 * (size_t)cells + cell] = sum[2] + sv;
+  acc[3 * (size_t)cells + cell] = sum[3] + sw;
+  acc[4 * (size_t)cells + cell] = sum[4] + se;
 }
 
 }  // namespace dev
