@@ -235,7 +235,7 @@ static __device__ __noinline__ void giant_cell(const StepParams& p, uint32_t cel
       if (active && !live) removed++;
       if (has_key) {
         const uint32_t key = cell_id3d(p.grid, pos.x, pos.y, pos.z);
-        warp_count_key(p.count, key, m, s_tile);
+        warp_count_key(p.count, key, s_tile);
         p.out_key[s + q] = key;
       } else if (active) {
         p.out_key[s + q] = kDeadKey;
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_cell(const __grid_constant__ 
             if (go && !live) removed++;
             if (has_key) {
               const uint32_t key = cell_id3d(p.grid, pos.x, pos.y, pos.z);
-              warp_count_key(p.count, key, m, s_tile);
+              warp_count_key(p.count, key, s_tile);
               p.out_key[g] = key;
             } else if (go) {
               p.out_key[g] = kDeadKey;

@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(WARPS * 32, 5) k_ntc_wb(const __grid_constant_
 // the streaming kernels count tiles in shared memory.
 __device__ __forceinline__ void finish_flight(const StepParams& p, bool go, bool live, uint32_t g,
                                               float3 pos, float3 vel, uint32_t& removed,
-                                              uint32_t* s_tile = nullptr) {
+                                              uint32_t* s_tile = nullptr, bool matched = false) {
   if (go) {
     p.out.x[g] = pos.x; p.out.y[g] = pos.y; p.out.z[g] = pos.z;
     p.out.u[g] = vel.x; p.out.v[g] = vel.y; p.out.w[g] = vel.z;
@@ -647,8 +647,10 @@ __device__ __forceinline__ void finish_flight(const StepParams& p, bool go, bool
     if (go && !live) removed++;
     if (has_key) {
       const uint32_t key = cell_id3d(p.grid, pos.x, pos.y, pos.z);
-      if (s_tile)
-        warp_count_key(p.count, key, m, s_tile);
+      if (s_tile && matched)
+        warp_count_key_matched(p.count, key, m, s_tile);
+      else if (s_tile)
+        warp_count_key(p.count, key, s_tile);
       else
         warp_count_key_global(p.count, key, m, p.tile_sum);
       p.out_key[g] = key;
@@ -688,6 +690,7 @@ __device__ __forceinline__ void flight_body(const StepParams& p, const uint32_t 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t step = p.step_override ? p.step_override : p.meta->step;
   const uint32_t n = p.meta->n_alive;
+  const bool matched = n >= kMatchedKeys * p.cells;
   const bool do_move = (p.flags & kDoMove) != 0;
   const bool split = p.has_geom && do_move;
   const bool piped = split && p.geom.nearest;
@@ -730,7 +733,7 @@ __device__ __forceinline__ void flight_body(const StepParams& p, const uint32_t 
     bool live = true;
     // a path that cannot reach the body
     if (go && do_move) live = move_free(p, pos, vel, g, step);
-    finish_flight(p, go, live, g, pos, vel, removed, s_tile);
+    finish_flight(p, go, live, g, pos, vel, removed, s_tile, matched);
     if (nq >= 32) {
       __syncwarp();
       nq -= 32;
@@ -835,7 +838,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_flight_pw(const __grid_con
         if (go && !live[k]) removed++;
         if (has_key) {
           key[k] = cell_id3d(p.grid, pos[k].x, pos[k].y, pos[k].z);
-          warp_count_key(p.count, key[k], m, s_tile);
+          warp_count_key(p.count, key[k], s_tile);
         }
       }
     }

@@ -89,8 +89,7 @@ __global__ void k_index(GridGeom g, const float* __restrict__ x, const float* __
       if (live) key = cell_id3d(g, px, py, pz);
       keys[i] = key;
     }
-    const unsigned m = __ballot_sync(kFull, active && live);
-    if (active && live) warp_count_key(count, key, m, s_tile);
+    if (active && live) warp_count_key(count, key, s_tile);
   }
   __syncthreads();
   flush_tile_hist(s_tile, tile_sum, n_scan_tiles);
@@ -330,7 +329,7 @@ __global__ void __launch_bounds__(256) k_count_keys(const uint32_t* __restrict__
     }
 #pragma unroll
     for (int k = 0; k < U; k++)
-      if (key[k] < nkeys) warp_count_key(count, key[k], 0u, s_tile);
+      if (key[k] < nkeys) warp_count_key(count, key[k], s_tile);
   }
   __syncthreads();
   flush_tile_hist(s_tile, tile_sum, n_scan_tiles);
@@ -850,8 +849,7 @@ __device__ __forceinline__ void inject_fill_body(const InjectParams& p, const ui
       p.st.u[d] = vel.x; p.st.v[d] = vel.y; p.st.w[d] = vel.z;
       p.keys[d] = key;
     }
-    const unsigned m = __ballot_sync(kFull, active && live);
-    if (active && live) warp_count_key(p.count, key, m, s_tile);
+    if (active && live) warp_count_key(p.count, key, s_tile);
   }
   __syncthreads();
   flush_tile_hist(s_tile, p.tile_sum, p.n_scan_tiles);
