@@ -1982,13 +1982,40 @@ void offsets(const std::vector<uint32_t>& blocks, std::vector<uint32_t>& out) {
   for (uint32_t k : blocks) out.push_back(out.back() + std::max(k, 1u));
 }
 
-// Shares of `wave` blocks by weight, at least one block each.
+// Shares of `wave` blocks by weight, at least one block each: whole blocks
+// first, then one at a time to the member with the most weight per block.
+// Never more than the wave where it holds a block for everyone (one block
+// too many starts when the others are nearly done: 285 us of the order kernel
+// of 32 members instead of 265).
 std::vector<uint32_t> shares(const std::vector<double>& w, uint32_t wave) {
   double total = 0.0;
   for (double x : w) total += x;
   std::vector<uint32_t> out(w.size(), 1u);
-  for (size_t i = 0; i < w.size(); i++)
-    if (total > 0.0) out[i] = std::max(1u, (uint32_t)std::lround((double)wave * w[i] / total));
+  if (!(total > 0.0)) return out;
+  uint32_t sum = 0;
+  for (size_t i = 0; i < w.size(); i++) {
+    out[i] = std::max(1u, (uint32_t)std::floor((double)wave * w[i] / total));
+    sum += out[i];
+  }
+  auto pick = [&](bool give) {
+    size_t at = w.size();
+    double best = 0.0;
+    for (size_t i = 0; i < w.size(); i++) {
+      if (!give && out[i] == 1u) continue;
+      const double load = w[i] / (double)(give ? out[i] : out[i] - 1u);
+      if (at == w.size() || (give ? load > best : load < best)) {
+        at = i;
+        best = load;
+      }
+    }
+    return at;
+  };
+  for (; sum < wave; sum++) out[pick(true)]++;
+  for (; sum > wave; sum--) {
+    const size_t i = pick(false);
+    if (i == w.size()) break;
+    out[i]--;
+  }
   return out;
 }
 
@@ -1996,9 +2023,9 @@ std::vector<uint32_t> shares(const std::vector<double>& w, uint32_t wave) {
 // members, member i running its own parameters in a share of the grid
 // (dsmcb::BatchOf), in the stage order of a member stepped alone (scan,
 // scatter, order, inflow injection, NTC, flight, mesh, sampling).  Shares
-// follow the members' particle counts at capture time (cells for the scan and
-// the sampling), so that every stage fills the GPU once with the whole
-// ensemble's work instead of once per member.
+// follow the members' particle counts and cells at capture time, so that
+// every stage fills the GPU once with the whole ensemble's work instead of
+// once per member.
 int batch_capture(dsmc_batch* b, const std::vector<float>& dt) {
   batch_drop_graph(b);
   const size_t n = b->members.size();
@@ -2039,19 +2066,25 @@ int batch_capture(dsmc_batch* b, const std::vector<float>& dt) {
   // inflow plan (one block per face) and fill
   std::vector<std::vector<uint32_t>> blocks(9);
   for (size_t i = 0; i < n; i++) blocks[0].push_back(b->members[i]->n_scan_tiles);
-  // the order kernel's and the NTC kernel's work per tile of 32 cells has a
-  // floor (a tile's chunk costs about as much with few particles as with
-  // eight per cell): weigh their shares by cells as well as particles
-  std::vector<double> wcell(n);
-  for (size_t i = 0; i < n; i++) wcell[i] = np[i] + 8.0 * nc[i];
-  blocks[1] = shares(np, (uint32_t)dsmcb::num_sms() * 4u);
-  blocks[2] = shares(wcell, wave[0]);
+  // Block times of members of 50,000 to 1,750,000 particles on 65,536 cells:
+  // a cell costs the order kernel as much as 3 particles, and its ranks grow
+  // with the square of a cell's particles; a cell costs the sampling as much
+  // as 12.  Weighed so, 32 members' order blocks end nearly together (by
+  // particles and 8 per cell: after 236 us on the average and 352 us at the
+  // longest, now 265).
+  std::vector<double> worder(n), wsample(n);
+  for (size_t i = 0; i < n; i++) {
+    worder[i] = np[i] + 3.0 * nc[i] + 0.02 * np[i] * np[i] / nc[i];
+    wsample[i] = np[i] + 12.0 * nc[i];
+  }
+  blocks[1] = shares(np, (uint32_t)dsmcb::num_sms() * 5u);
+  blocks[2] = shares(worder, wave[0]);
   for (size_t i = 0; i < n; i++)  // the order kernel needs no more warps than tiles
     blocks[2][i] = std::min(blocks[2][i], std::max(1u, (P[i].n_tiles + 3u) / 4u));
-  blocks[3] = shares(wcell, wave[1]);
+  blocks[3] = shares(np, wave[1]);  // the NTC kernel cuts its grid by itself
   blocks[4] = shares(np, wave[2]);
   blocks[5] = shares(np, wave[3]);
-  blocks[6] = shares(nc, wave[4]);
+  blocks[6] = shares(wsample, wave[4]);
   blocks[7].assign(I.size(), 1u);
   blocks[8].assign(I.size(), 4u);
   std::vector<uint32_t> off;

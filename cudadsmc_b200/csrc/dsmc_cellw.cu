@@ -617,12 +617,52 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_ntc_w(const __grid_constant__
   chained_entry();
   ntc_body<WARPS>(p, blockIdx.x, gridDim.x);
 }
+// The NTC kernel's share of a batched grid: one block per member and the rest
+// by the members' listed work (32 light cells or one dense cell each take a
+// warp about 6 us).  It follows the members' speeds and mean free paths as
+// much as their sizes, and is known only now: shares by particles and cells
+// left 32 sphere flows' blocks done after 28 us on the average and 99 us at
+// the longest.  Each warp sums the lists for itself (a few loads that all
+// blocks share in L2).  false: a block that the rounding left over.
+__device__ __forceinline__ bool ntc_share(const BatchOf<StepParams>& bv, uint32_t& member, uint32_t& vb,
+                                          uint32_t& vg) {
+  const uint32_t lane = lane_id();
+  auto work = [&](uint32_t m) {
+    const Meta* t = m < bv.members ? bv.items[m].meta : nullptr;
+    return t ? (t->n_light + 31u) / 32u + t->n_heaviest + t->n_heavy : 0u;
+  };
+  uint64_t total = 0;
+  for (uint32_t m = lane; m < bv.members; m += 32) total += work(m);
+  total = warp_sum(total);
+  const uint64_t spare = gridDim.x - bv.members;
+  uint32_t first = 0;
+  for (uint32_t m0 = 0; m0 < bv.members; m0 += 32) {
+    const uint32_t m = m0 + lane;
+    const uint32_t mine = m < bv.members ? 1u + (total ? (uint32_t)(spare * work(m) / total) : 0u) : 0u;
+    uint32_t end = mine;
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t up = __shfl_up_sync(kFull, end, d);
+      if (lane >= (uint32_t)d) end += up;
+    }
+    const uint32_t b = blockIdx.x - first;  // this block among these members' ones
+    const unsigned in = __ballot_sync(kFull, b >= end - mine && b < end);
+    if (in) {
+      const int l = __ffs(in) - 1;
+      member = m0 + (uint32_t)l;
+      vg = __shfl_sync(kFull, mine, l);
+      vb = b - (__shfl_sync(kFull, end, l) - vg);
+      return true;
+    }
+    first += __shfl_sync(kFull, end, 31);
+  }
+  return false;
+}
+
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 5) k_ntc_wb(const __grid_constant__ BatchOf<StepParams> bv) {
   chained_entry();
-  uint32_t vb, vg;
-  const StepParams& p = bv.locate(vb, vg);
-  ntc_body<WARPS>(p, vb, vg);
+  uint32_t member, vb, vg;
+  if (ntc_share(bv, member, vb, vg)) ntc_body<WARPS>(bv.items[member], vb, vg);
 }
 
 // ------------------------------------------------ flight + keys + sample ----
@@ -1358,7 +1398,7 @@ cudaError_t cell_batch_waves(uint32_t wave[5], size_t flight_smem) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_flight_wb<kFlightWarps, 4>, kFlightWarps * 32,
                                                       flight_smem);
   if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[3], k_mesh_wb<2, true>, 32 * kMeshWarps, 0);
-  per[4] = 8;
+  per[4] = 8;  // more than a wave of sampling blocks: 3 per SM ran the ensemble's steps 11 us longer
   if (e != cudaSuccess) return e;
   for (int k = 0; k < 5; k++) {
     if (per[k] < 1) return cudaErrorInvalidConfiguration;
