@@ -413,8 +413,12 @@ __device__ __forceinline__ void order_body(const StepParams& p, const uint32_t v
           p.maxrem[gc] = vm;
           sel += M;
         }
-        buffer_cells(S.lbuf, lcnt, p.ntc_light, &p.meta->n_light, lane == C.cur && M > 0,
+        // (in the Philox mode to a warp's, among the first to start)
+        const bool warp_cell = heavy_mode && M >= kHeavyMin && M < kGiantPairs;
+        buffer_cells(S.lbuf, lcnt, p.ntc_light, &p.meta->n_light, lane == C.cur && M > 0 && !warp_cell,
                      make_uint4(gc, C.base, C.n, M));
+        list_cells(p.ntc_heavy, 1, &p.meta->n_heaviest, lane == C.cur && warp_cell,
+                   make_uint4(gc, C.base, C.n, M | kGiantPairs));
       }
     } else if (C.n > 0) {
       // a pending chunk in this chunk's buffer (an empty chunk came between)
@@ -516,7 +520,7 @@ constexpr uint32_t kNtcClaim = 256;  // claim slots per warp: the largest chunk
 
 // The NTC selections of the cells k_order_w listed, in place on the sorted
 // post-collision state p.mid: a lane per light cell, a warp per dense cell
-// (at most kNtcClaim particles: larger cells were collided by k_order_w).
+// and per cell above the chunk (ntc_select_fast_warp).
 // The pair counts and remainders come from k_order_w; this kernel updates
 // (sigma g)max (and the HybridTaus state in the reference RNG mode) with the
 // same arithmetic and random streams as the fused path.  The grid is one
@@ -565,18 +569,26 @@ __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb,
       float* su = s_vel[warp][0];
       float* sv = s_vel[warp][1];
       float* sw = s_vel[warp][2];
-      for (uint32_t t = lane; t < e.z; t += 32) {
+      // (but for a cell above the chunk that does not fit)
+      const bool fits = e.z <= kNtcClaim;
+      for (uint32_t t = lane; fits && t < e.z; t += 32) {
         su[t] = p.mid.u[e.y + t];
         sv[t] = p.mid.v[e.y + t];
         sw[t] = p.mid.w[e.y + t];
       }
       const float2 vm = p.maxrem[e.x];  // .y: the remainder k_order_w stored
       __syncwarp();
-      GlobalVel acc{su, sv, sw, 0u};
-      const float vmax =
-          ntc_select_heavy_warp(p, e.x, e.z, acc, s_claim[warp], step, e.w, vm.x, col, sum_g);
+      float vmax;
+      if (e.w & kGiantPairs) {
+        const GlobalVel acc = fits ? GlobalVel{su, sv, sw, 0u} : GlobalVel{p.mid.u, p.mid.v, p.mid.w, e.y};
+        vmax = ntc_select_fast_warp(p, e.x, e.z, acc, s_claim[warp], step, e.w & ~kGiantPairs, vm.x, col, sum_g);
+        for (uint32_t t = lane; t < 128u; t += 32) s_claim[warp][t] = 0xffffffffu;
+      } else {
+        const GlobalVel acc{su, sv, sw, 0u};
+        vmax = ntc_select_heavy_warp(p, e.x, e.z, acc, s_claim[warp], step, e.w, vm.x, col, sum_g);
+      }
       __syncwarp();
-      for (uint32_t t = lane; t < e.z; t += 32) {
+      for (uint32_t t = lane; fits && t < e.z; t += 32) {
         p.mid.u[e.y + t] = su[t];
         p.mid.v[e.y + t] = sv[t];
         p.mid.w[e.y + t] = sw[t];
