@@ -581,7 +581,7 @@ __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb,
       float vmax;
       if (e.w & kGiantPairs) {
         const GlobalVel acc = fits ? GlobalVel{su, sv, sw, 0u} : GlobalVel{p.mid.u, p.mid.v, p.mid.w, e.y};
-        vmax = ntc_select_fast_warp(p, e.x, e.z, acc, s_claim[warp], step, e.w & ~kGiantPairs, vm.x, col, sum_g);
+        vmax = ntc_select_fast_warp(p, e.x, e.z, acc, reinterpret_cast<float*>(s_claim[warp]), step, e.w & ~kGiantPairs, vm.x, col, sum_g);
         for (uint32_t t = lane; t < 128u; t += 32) s_claim[warp][t] = 0xffffffffu;
       } else {
         const GlobalVel acc{su, sv, sw, 0u};

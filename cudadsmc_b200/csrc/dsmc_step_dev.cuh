@@ -449,75 +449,75 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
 // ntc_select_fast's selections of one cell by a whole warp, the same pairs,
 // numbers and order of results: for the cells above a chunk, which one lane
 // would hold the NTC kernel up with (0.7 us a pair: 77 us for the kernel of an
-// ensemble of 32 sphere flows, 50 us with a warp).  The pairs do not
-// depend on the collisions, so each lane draws and evaluates one of the next
-// 32.  What is sequential is the place of a pair's numbers in the collision
-// stream (three words after a collision, one otherwise) and (sigma g)max: a
-// short walk over the evaluated pairs finds both, up to the first pair that
-// has a particle of a collision before it; then the collisions walked over
-// are carried out side by side, and the pair that ended the walk is the next
-// first.  words: 128 words of shared memory for the numbers of 32 pairs.
+// ensemble of 32 sphere flows; 0.2 us here).  The pairs do not
+// depend on the collisions, so each lane draws one of the next 32 and
+// evaluates it.  What is sequential is the place of a pair's numbers in the
+// collision stream (three words after a collision, one otherwise) and (sigma
+// g)max: a short walk over the evaluated pairs finds both, up to the first
+// pair that has a particle of a collision of this walk; then the collisions
+// walked over are carried out side by side, and the pairs from there on are
+// evaluated again.  numbers: 128 floats of shared memory for the numbers of
+// 32 pairs.
 template <class Acc>
-__device__ __noinline__ float ntc_select_fast_warp(const StepParams& p, uint32_t cell, uint32_t n, Acc acc,
-                                                      uint32_t* words, uint32_t step, uint32_t M, float vmax,
+__device__ __forceinline__ float ntc_select_fast_warp(const StepParams& p, uint32_t cell, uint32_t n, Acc acc,
+                                                      float* numbers, uint32_t step, uint32_t M, float vmax,
                                                       uint32_t& col, double& sum_g) {
   const uint32_t lane = lane_id();
   uint32_t pos = 0;  // of the next pair's numbers in the collision stream
-  for (uint32_t k = 0; k < M;) {
+  for (uint32_t k = 0; k < M; k += 32) {
     const uint32_t cnt = min(32u, M - k), mine = k + lane;
     const uint4 q = philox4x32_10(make_uint4(mine >> 1, cell, step, kPurposePairs), p.seed);
     const uint32_t pi = __umulhi((mine & 1u) ? q.z : q.x, n);
     uint32_t pj = pi + 1u + __umulhi((mine & 1u) ? q.w : q.y, n - 1u);
     if (pj >= n) pj -= n;
-    const float3 v1 = acc.get(pi), v2 = acc.get(pj);
     const uint32_t w0 = pos & ~3u;
     const uint4 w = philox4x32_10(make_uint4((w0 >> 2) + lane, cell, step, kPurposeCollide), p.seed);
+    auto uniform = [](uint32_t x) { return ((float)(x >> 8) + 0.5f) * (1.0f / 16777216.0f); };
+    numbers[4 * lane] = uniform(w.x);
+    numbers[4 * lane + 1] = uniform(w.y);
+    numbers[4 * lane + 2] = uniform(w.z);
+    numbers[4 * lane + 3] = uniform(w.w);
     __syncwarp();
-    words[4 * lane] = w.x;
-    words[4 * lane + 1] = w.y;
-    words[4 * lane + 2] = w.z;
-    words[4 * lane + 3] = w.w;
-    auto uniform = [&](uint32_t at) {
-      return ((float)(words[at - w0] >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    };
-    const float mag = rel_speed(v1, v2);
-    const float v = lane < cnt ? sigma_g_fast(p, mag) : 0.f;
-    // the earlier pairs that share a particle with this one, and (sigma g)max
-    // before it
-    uint32_t shared = 0;
+    const float* num = numbers - w0;
+    uint32_t shared = 0;  // the earlier pairs that have a particle of this one
     for (uint32_t l = 0; l < 31; l++) {
       const uint32_t a = __shfl_sync(kFull, pi, l), b = __shfl_sync(kFull, pj, l);
       if (l < lane && (a == pi || a == pj || b == pi || b == pj)) shared |= 1u << l;
     }
-    float top = v;  // over this lane's pair and the ones before it
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-      const float up = __shfl_up_sync(kFull, top, d);
-      if (lane >= d) top = fmaxf(top, up);
+    for (uint32_t c = 0; c < cnt;) {
+      const float3 v1 = acc.get(pi), v2 = acc.get(pj);
+      const float mag = rel_speed(v1, v2);
+      const float v = lane >= c && lane < cnt ? sigma_g_fast(p, mag) : 0.f;
+      float top = v;  // (sigma g)max after this lane's pair
+      for (uint32_t d = 1; d < 32; d <<= 1) {
+        const float up = __shfl_up_sync(kFull, top, d);
+        if (lane >= d) top = fmaxf(top, up);
+      }
+      top = fmaxf(vmax, top);
+      float before = __shfl_up_sync(kFull, top, 1);
+      if (lane == 0) before = vmax;
+      uint32_t hit = 0, got = c, at = pos;
+      for (; got < cnt; got++) {
+        if (__shfl_sync(kFull, shared, got) & hit) break;
+        const bool yes = __shfl_sync(kFull, v, got) > num[at] * __shfl_sync(kFull, before, got);
+        if (yes) hit |= 1u << got;
+        at += yes ? 3u : 1u;
+      }
+      __syncwarp();
+      if ((hit >> lane) & 1u) {
+        const uint32_t own = pos + (lane - c) + 2u * __popc(hit & ((1u << lane) - 1u));
+        col++;
+        sum_g += mag;
+        float3 o1, o2;
+        scatter_pair(v1, v2, mag, num[own + 1u], num[own + 2u], o1, o2);
+        acc.set(pi, o1);
+        acc.set(pj, o2);
+      }
+      vmax = __shfl_sync(kFull, top, got - 1u);
+      pos = at;
+      c = got;
+      __syncwarp();
     }
-    top = fmaxf(vmax, top);
-    float before = __shfl_up_sync(kFull, top, 1);
-    if (lane == 0) before = vmax;
-    __syncwarp();
-    uint32_t hit = 0, got = 0, at = pos;
-    for (; got < cnt; got++) {
-      if (__shfl_sync(kFull, shared, got) & hit) break;
-      const bool yes = __shfl_sync(kFull, v, got) > uniform(at) * __shfl_sync(kFull, before, got);
-      if (yes) hit |= 1u << got;
-      at += yes ? 3u : 1u;
-    }
-    if ((hit >> lane) & 1u) {
-      const uint32_t own = pos + lane + 2u * __popc(hit & ((1u << lane) - 1u));
-      col++;
-      sum_g += mag;
-      float3 o1, o2;
-      scatter_pair(v1, v2, mag, uniform(own + 1u), uniform(own + 2u), o1, o2);
-      acc.set(pi, o1);
-      acc.set(pj, o2);
-    }
-    vmax = __shfl_sync(kFull, top, got - 1u);
-    pos = at;
-    k += got;
-    __syncwarp();
   }
   return vmax;
 }
