@@ -89,6 +89,12 @@ class Mlp(ctypes.Structure):
         ("mean", _P)]
 
 
+class AdamParam(ctypes.Structure):
+    """dsmc_adam_param"""
+    _fields_ = [(k, _P) for k in ("w", "g", "m", "v", "w_bf16")] + [("n", ctypes.c_size_t),
+                                                                     ("weight_decay", ctypes.c_float)]
+
+
 SIGNATURES = [
     ("dsmc_config_default", _I, [ctypes.POINTER(Config)]),
     ("dsmc_config_read_xml", _I, [ctypes.c_char_p, ctypes.POINTER(Config)]),
@@ -143,6 +149,8 @@ SIGNATURES = [
     ("dsmc_mse_grad", _I, [_P, _P, ctypes.c_size_t, ctypes.c_float, _P, _P, _P, _P, _P]),
     ("dsmc_adam_step", _I, [_P, _P, _P, _P, _P, ctypes.c_size_t, ctypes.c_float, ctypes.c_float,
                             ctypes.c_float, ctypes.c_float, _I, ctypes.c_float, _P]),
+    ("dsmc_adam_steps", _I, [_P, _I, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float, _I, _P]),
+    ("dsmc_layer_backward", _I, [_I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P]),
     ("dsmc_to_bf16", _I, [_P, _P, ctypes.c_size_t, _P]),
     ("dsmc_set_kernel_variant", _I, [_P, _I]),
     ("dsmc_get_kernel_variant", _I, [_P, _P, _P]),

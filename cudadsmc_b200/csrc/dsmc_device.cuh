@@ -271,6 +271,20 @@ __device__ __forceinline__ void chained_entry() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The same for a kernel that may run beside the one before it (`beside`: it
+// reads and writes nothing that the one before it writes, and nothing that
+// one reads is written by it).  What came before that one is complete when
+// its blocks have begun, so this kernel begins at once; its blocks end after
+// the one before is complete (beside_exit, which every thread passes), so
+// whatever waits for this kernel has waited for both.
+__device__ __forceinline__ void beside_entry(bool beside) {
+  if (!beside) asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void beside_exit(bool beside) {
+  if (beside) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Geometry on the device: the uniform grid over the body, a per-cell flag,
 // per-cell [start,end) into the bin entries, and per bin entry the three
 // vertices with the face normal packed into the .w lanes.

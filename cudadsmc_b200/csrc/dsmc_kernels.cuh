@@ -61,6 +61,9 @@ inline cudaError_t launch_chained(void (*kernel)(KArgs...), uint32_t grid, uint3
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// dsmc_colsum's kernel beside the one before it on the stream (beside_entry).
+cudaError_t launch_colsum_beside(const float* x, int rows, int cols, int ld, float* out, cudaStream_t stream);
+
 constexpr int kMaxCellsPerTile = 256;
 constexpr int kScanTile = 2048;       // cells per scan block (256 threads x 8)
 constexpr int kScanShift = 11;

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "dsmc_b200.h"
+#include "dsmc_kernels.cuh"
 
 namespace {
 
@@ -30,7 +31,9 @@ __global__ void k_gelu_backward(const float* z, const float* dh, float* dz, bf16
 // for each group of loads in turn, on two blocks for a layer's 512 columns:
 // 1024 x 512 61 us, now 10 us).
 constexpr int kColWarps = 8, kColRows = 128;
-__global__ void __launch_bounds__(32 * kColWarps) k_colsum(const float* x, int rows, int cols, int ld, float* out) {
+__global__ void __launch_bounds__(32 * kColWarps) k_colsum(const float* x, int rows, int cols, int ld, float* out,
+                                                           bool beside) {
+  dsmcb::beside_entry(beside);
   __shared__ float st[2][kColRows][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
@@ -62,6 +65,7 @@ __global__ void __launch_bounds__(32 * kColWarps) k_colsum(const float* x, int r
     }
   }
   if (w == 0 && col < cols) out[col] = s;
+  dsmcb::beside_exit(beside);
 }
 
 // Masked MSE: targets that are NaN carry no loss.  dy = scale * 2 (y - t).
@@ -122,7 +126,9 @@ __device__ __forceinline__ void adam_one(const AdamArgs& a, float gi, float& w, 
 // 84M weights 558 -> 400 us, 0.96 of the copy bandwidth.
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_adam(float* w, const float* g, float* m, float* v, bf16* wb, size_t n,
-                                              const AdamArgs a) {
+                                              const AdamArgs a,
+                                              bool beside) {
+  dsmcb::beside_entry(beside);
   const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
   size_t done = 0;
   if (VEC) {
@@ -150,6 +156,7 @@ __global__ void __launch_bounds__(256) k_adam(float* w, const float* g, float* m
     adam_one(a, g[i], w[i], m[i], v[i]);
     if (wb) wb[i] = __float2bfloat16(w[i]);
   }
+  dsmcb::beside_exit(beside);
 }
 
 __global__ void k_to_bf16(const float* x, bf16* y, size_t n) {
@@ -166,6 +173,11 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 }  // namespace
 
+cudaError_t dsmcb::launch_colsum_beside(const float* x, int rows, int cols, int ld, float* out, cudaStream_t stream) {
+  return launch_chained(k_colsum, (uint32_t)(cols + 31) / 32, 32 * kColWarps, 0, stream, true, x, rows, cols, ld, out,
+                        true);
+}
+
 extern "C" {
 
 int dsmc_gelu_backward(const float* z, const float* dh, float* dz, void* dz_bf16, size_t n,
@@ -177,7 +189,7 @@ int dsmc_gelu_backward(const float* z, const float* dh, float* dz, void* dz_bf16
 
 int dsmc_colsum(const float* x, int rows, int cols, int ld, float* out, void* stream) {
   if (!x || !out || rows < 0 || cols <= 0) return DSMC_ERR_ARG;
-  k_colsum<<<(cols + 31) / 32, 32 * kColWarps, 0, (cudaStream_t)stream>>>(x, rows, cols, ld, out);
+  k_colsum<<<(cols + 31) / 32, 32 * kColWarps, 0, (cudaStream_t)stream>>>(x, rows, cols, ld, out, false);
   return cudaGetLastError() == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
 }
 
@@ -189,16 +201,32 @@ int dsmc_mse_grad(const float* y, const void* t_bf16, size_t n, float scale, voi
   return cudaGetLastError() == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
 }
 
-int dsmc_adam_step(float* w, const float* g, float* m, float* v, void* w_bf16, size_t n, float lr,
-                   float b1, float b2, float eps, int t, float weight_decay, void* stream) {
+static int adam(float* w, const float* g, float* m, float* v, void* w_bf16, size_t n, float lr, float b1, float b2,
+                float eps, int t, float weight_decay, bool beside, void* stream) {
   if (!w || !g || !m || !v || t < 1) return DSMC_ERR_ARG;
   AdamArgs a{lr, b1, b2, eps, 1.f - powf(b1, (float)t), 1.f - powf(b2, (float)t), weight_decay};
   bf16* wb = static_cast<bf16*>(w_bf16);
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = aligned16(w) && aligned16(g) && aligned16(m) && aligned16(v) && ((uintptr_t)wb & 7u) == 0;
-  if (vec) k_adam<true><<<grid_1d((n + 3) / 4), 256, 0, s>>>(w, g, m, v, wb, n, a);
-  else k_adam<false><<<grid_1d(n), 256, 0, s>>>(w, g, m, v, wb, n, a);
-  return cudaGetLastError() == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
+  const cudaError_t e = dsmcb::launch_chained(vec ? k_adam<true> : k_adam<false>, grid_1d(vec ? (n + 3) / 4 : n), 256, 0, s,
+                                              beside, w, g, m, v, wb, n, a, beside);
+  return e == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
+}
+
+int dsmc_adam_step(float* w, const float* g, float* m, float* v, void* w_bf16, size_t n, float lr,
+                   float b1, float b2, float eps, int t, float weight_decay, void* stream) {
+  return adam(w, g, m, v, w_bf16, n, lr, b1, b2, eps, t, weight_decay, false, stream);
+}
+
+int dsmc_adam_steps(const dsmc_adam_param* params, int count, float lr, float b1, float b2, float eps, int t,
+                    void* stream) {
+  if (!params || count < 0) return DSMC_ERR_ARG;
+  for (int i = 0; i < count; i++) {
+    const dsmc_adam_param& p = params[i];
+    const int st = adam(p.w, p.g, p.m, p.v, p.w_bf16, p.n, lr, b1, b2, eps, t, p.weight_decay, i > 0, stream);
+    if (st != DSMC_OK) return st;
+  }
+  return DSMC_OK;
 }
 
 int dsmc_to_bf16(const float* x, void* y, size_t n, void* stream) {

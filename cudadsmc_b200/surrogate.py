@@ -15,7 +15,7 @@ import math
 
 import numpy as np
 
-from ._capi import Mlp, check, lib
+from ._capi import AdamParam, Mlp, check, lib
 
 _P = ctypes.c_void_p
 
@@ -119,6 +119,17 @@ class WarmStartMLP:
         return self._forward(x, cache=True, field=True)
 
     # ----------------------------------------------------------- backward --
+    def _layer_backward(self, g, w, b, x, dz, dzb, inner):
+        """The gradients of weights w and bias b into g; returns the input's (`inner`) or None."""
+        B, dout = dz.shape
+        din = x.shape[1]
+        g[w] = self.torch.empty((din, dout), dtype=self.torch.float32, device=self.dev)
+        g[b] = self.torch.empty(dout, dtype=self.torch.float32, device=self.dev)
+        dx = self.torch.empty((B, din), dtype=self.torch.float32, device=self.dev) if inner else None
+        check(lib().dsmc_layer_backward(B, din, dout, _p(x), _p(dz), _p(dzb), _p(self.bf[w]), _p(g[w]), _p(g[b]),
+                                        _p(dx), _stream()), "layer_backward")
+        return dx
+
     def loss_and_grads(self, x, targets_bf16):
         """Masked MSE against BF16 targets [batch, F] (NaN = no target).
         Returns (loss, valid count, grads dict of FP32 tensors)."""
@@ -144,40 +155,23 @@ class WarmStartMLP:
                          device=self.dev)
         check(lib().dsmc_gemm_split_bf16(B, self.modes, self.F, _p(dyb), self.F, 0, _p(self.bf["B"]), self.F, 1,
                                          _p(dc), _p(dcb), split, _p(ws), _stream()), "gemm_split_bf16")
-        g["Wout"] = torch.empty((self.hidden, self.modes), dtype=torch.float32, device=self.dev)
-        self._gemm(self.hidden, self.modes, B, cache["h"], self.hidden, 1, dcb, self.modes, 0, g["Wout"],
-                   self.modes)
-        g["bout"] = torch.empty(self.modes, dtype=torch.float32, device=self.dev)
-        check(lib().dsmc_colsum(_p(dc), B, self.modes, self.modes, _p(g["bout"]), _stream()), "colsum")
-        dh = torch.empty((B, self.hidden), dtype=torch.float32, device=self.dev)
-        self._gemm(B, self.hidden, self.modes, dcb, self.modes, 0, self.bf["Wout"], self.modes, 1, dh,
-                   self.hidden)
+        dh = self._layer_backward(g, "Wout", "bout", cache["h"], dc, dcb, True)
         for l in range(self.depth - 1, -1, -1):
             z = cache["z"][l]
             dz = torch.empty_like(z)
             dzb = torch.empty(z.shape, dtype=torch.bfloat16, device=self.dev)
             check(lib().dsmc_gelu_backward(_p(z), _p(dh), _p(dz), _p(dzb), z.numel(), _stream()),
                   "gelu_backward")
-            xin = cache["x"][l]
-            din = xin.shape[1]
-            g[f"W{l}"] = torch.empty((din, self.hidden), dtype=torch.float32, device=self.dev)
-            self._gemm(din, self.hidden, B, xin, din, 1, dzb, self.hidden, 0, g[f"W{l}"], self.hidden)
-            g[f"b{l}"] = torch.empty(self.hidden, dtype=torch.float32, device=self.dev)
-            check(lib().dsmc_colsum(_p(dz), B, self.hidden, self.hidden, _p(g[f"b{l}"]), _stream()),
-                  "colsum")
-            if l > 0:
-                dh = torch.empty((B, din), dtype=torch.float32, device=self.dev)
-                self._gemm(B, din, self.hidden, dzb, self.hidden, 0, self.bf[f"W{l}"], self.hidden, 1, dh,
-                           din)
+            dh = self._layer_backward(g, f"W{l}", f"b{l}", cache["x"][l], dz, dzb, l > 0)
         return acc, cnt, g, y
 
     def adam_step(self, grads, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8, weight_decay=0.0):
         self.t += 1
-        for k, w in self.params.items():
-            check(lib().dsmc_adam_step(_p(w), _p(grads[k]), _p(self.m[k]), _p(self.v[k]),
-                                       _p(self.bf.get(k)), w.numel(), lr, b1, b2, eps, self.t,
-                                       weight_decay if k.startswith("W") else 0.0, _stream()),
-                  "adam_step")
+        ps = (AdamParam * len(self.params))(*[
+            AdamParam(*(_p(a) for a in (w, grads[k], self.m[k], self.v[k], self.bf.get(k))), w.numel(),
+                      weight_decay if k.startswith("W") else 0.0)
+            for k, w in self.params.items()])
+        check(lib().dsmc_adam_steps(ps, len(ps), lr, b1, b2, eps, self.t, _stream()), "adam_steps")
 
     def train(self, x, targets_bf16, epochs=200, batch=128, lr=1e-3, lr_final=1e-5, seed=0,
               log=None):

@@ -577,6 +577,13 @@ int dsmc_gelu_backward(const float* z, const float* dh, float* dz, void* dz_bf16
                        void* stream);
 /* out[col] = sum over rows of x[row * ld + col]. */
 int dsmc_colsum(const float* x, int rows, int cols, int ld, float* out, void* stream);
+/* A layer's gradients from dz (batch x dout, FP32 and the same in BF16), its
+ * BF16 input x (batch x din) and weights w (din x dout): dw = x^T dz, db the
+ * column sums of dz and, unless dx is NULL, dx = dz w^T.  Arrays without
+ * padding; the conditions of dsmc_gemm_bf16.  The three run side by side:
+ * none of the outputs may overlap an input or another output. */
+int dsmc_layer_backward(int batch, int din, int dout, const void* x, const float* dz, const void* dz_bf16,
+                        const void* w, float* dw, float* db, float* dx, void* stream);
 /* Masked mean-square error: for every finite BF16 target t, loss += (y - t)^2,
  * count += 1 and dy = scale * 2 (y - t); NaN targets give dy = 0. */
 int dsmc_mse_grad(const float* y, const void* t_bf16, size_t n, float scale, void* dy_bf16, float* dy,
@@ -584,6 +591,19 @@ int dsmc_mse_grad(const float* y, const void* t_bf16, size_t n, float scale, voi
 /* Adam step t (>= 1) with decoupled weight decay; refreshes w_bf16 if given. */
 int dsmc_adam_step(float* w, const float* g, float* m, float* v, void* w_bf16, size_t n, float lr,
                    float b1, float b2, float eps, int t, float weight_decay, void* stream);
+/* dsmc_adam_step for `count` parameters, which may run side by side: their
+ * arrays are distinct. */
+typedef struct dsmc_adam_param {
+  float* w;
+  const float* g;
+  float* m;
+  float* v;
+  void* w_bf16; /* or NULL */
+  size_t n;
+  float weight_decay;
+} dsmc_adam_param;
+int dsmc_adam_steps(const dsmc_adam_param* params, int count, float lr, float b1, float b2, float eps, int t,
+                    void* stream);
 int dsmc_to_bf16(const float* x, void* y, size_t n, void* stream);
 
 #ifdef __cplusplus
