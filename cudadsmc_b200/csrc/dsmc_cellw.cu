@@ -15,11 +15,12 @@
 //   B  NTC pair counts (and remainders); cells with pairs are listed
 //   C  the chunk goes to the mid arrays in sorted order
 // k_ntc_w: the listed cells' NTC selections in place on the mid arrays, a
-// lane per light cell, a warp per dense cell (Philox mode).
+// lane per light cell, a warp per dense cell and per cell above a chunk
+// (Philox mode).
 // k_flight_w (flight + keys): streams the sorted particles, 32 at a time per
-// warp in grid-stride order: free flight and boundaries, next-step key and
-// count (warp-aggregated atomics on the per-cell counts and on the per scan
-// tile totals).  Flights that may reach the body are listed instead: they
+// warp, each warp a contiguous run: free flight and boundaries, next-step key
+// and count (atomics on the per-cell counts and on the block's histogram of
+// scan tile totals).  Flights that may reach the body are listed instead: they
 // cluster next to the body, so k_mesh_w flies them afterwards one per thread
 // over the whole GPU.  k_sample_w samples (FP64) on sampling steps.
 //

@@ -307,13 +307,12 @@ int dsmc_step_graph(dsmc_handle* h, float dt, int nsteps);
  * whose kernels use fixed block sizes).  Variants 0-3 are a CTA-wide kernel:
  * 0 = 512 threads per CTA and up to 2048 particles per shared-memory chunk,
  * 1 = 256/1024, 2 = 128/512, 3 = 64/256.  Variants 4-7 are split kernels
- * whose warps each work through their own tiles of 32 cells, with chunks of
- * up to 256 (4) or 128 (5-7) particles per warp; 5 is the default.  Results
- * do not
- * depend on the variant, except in the Philox mode for a cell holding more
- * particles than the chunk (it is then collided by one thread instead of one
- * warp, a different but equivalent stream of draws).  Changing it drops the
- * captured graph. */
+ * whose warps each work through their own tiles of 4 to 32 cells, with chunks
+ * of up to 256 (4) or 128 (5-7) particles per warp; 5 is the default.
+ * Results do not depend on the variant, except in the Philox mode for a cell
+ * holding more particles than the chunk (its selections then follow one after
+ * the other, with a different but equivalent stream of draws).  Changing it
+ * drops the captured graph. */
 int dsmc_set_kernel_variant(dsmc_handle* h, int variant);
 int dsmc_get_kernel_variant(dsmc_handle* h, int* variant, int* chunk_capacity);
 /* Number of cell-kernel variants (valid variants are 0 .. count-1). */
