@@ -223,7 +223,7 @@ void set_vhs_fast(dsmcb::StepParams& p, float cross_section, float omega, float 
 }
 
 // One shared-memory share for a step's kernels (Chain) where the order kernel's
-// tiles fit one wave of 16 warps per SM, which that share holds; the driver's
+// tiles fit one wave of 16 warps per SM, which that share holds; CUDA's own
 // choice elsewhere.
 int step_carveout(const dsmc_handle* h) {
   return dsmcb::cell_kernel_is_warp(h->variant) && dsmcb::cell_kernel_chunk_capacity(h->variant) == 128 &&

@@ -28,7 +28,7 @@ namespace dsmcb {
 // they save (1.78 against 2.10 ms per step of the 64-member ensemble), while
 // a single instance gains about 1 %.
 //
-// carveout (percent, -1: the driver's choice per kernel): the share of an
+// carveout (percent, -1: CUDA's own choice per kernel): the share of an
 // SM's memory set up as shared.  Kernels with different shares cannot be on
 // an SM together, so the next one's early CTAs wait for the one before to
 // leave; where a step's kernels are short, one share for all of them lets
