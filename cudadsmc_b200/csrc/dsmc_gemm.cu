@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
             if (g.tma_cb) tma_store(&map_cb, hst + 2048 * buf, c0, row0);
             bulk_commit();
           }
-          buf ^= 1;
+          buf = (buf + 1) % Sh::kStaging;  // the other block, where the warp has two
         }
       }
     }
