@@ -1220,6 +1220,7 @@ int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_
   dsmcb::SeedParams sp{};
   sp.fields = (const float*)w;
   sp.cells = h->cells;
+  sp.capacity = h->capacity;
   sp.frac = geo ? fill_frac(h) : nullptr;
   sp.cell_volume = h->cell_volume;
   sp.fnum = c.fnum;
@@ -1243,7 +1244,7 @@ int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_
   CK(h, cudaMemcpyAsync(&tot, sp.totals, sizeof(tot), cudaMemcpyDeviceToHost, h->stream), "seed totals");
   CK(h, cudaStreamSynchronize(h->stream), "seed totals");
   const uint64_t n = tot.n;
-  const uint32_t kmax = tot.kmax;
+  const uint32_t kmax = tot.kmax;  // <= n: the sum is exact
   if (n > h->capacity) return fail(h, DSMC_ERR_CAPACITY, "initial particles exceed capacity");
   CK(h, cudaMemcpyAsync(h->maxrem, sp.maxrem, nc * sizeof(float2), cudaMemcpyDeviceToDevice, h->stream),
      "seed collision state");

@@ -290,7 +290,7 @@ struct SeedTotals {
 };
 struct SeedParams {
   const float* fields;   // per cell n, u, v, w, T
-  uint32_t cells;
+  uint32_t cells, capacity;
   const float* frac;     // fraction of the cell outside the body (null: all 1)
   float cell_volume, fnum, temp, wall_temp, kb_m, max_rel_vel, weight;
   float stream[3];

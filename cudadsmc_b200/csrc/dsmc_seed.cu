@@ -52,7 +52,8 @@ constexpr int kThreads = 128;
 static_assert(kScanTile % kThreads == 0, "a block lies in one scan tile");
 
 __global__ void __launch_bounds__(kThreads) k_seed_cells(const SeedParams p) {
-  __shared__ uint32_t s_sum[kThreads / 32], s_max[kThreads / 32];
+  __shared__ unsigned long long s_sum[kThreads / 32];
+  __shared__ uint32_t s_max[kThreads / 32];
   const uint32_t cell = blockIdx.x * kThreads + threadIdx.x;
   uint32_t k = 0;
   if (cell < p.cells) {
@@ -60,8 +61,11 @@ __global__ void __launch_bounds__(kThreads) k_seed_cells(const SeedParams p) {
     // n is averaged over the whole cell volume (as dsmc_read_fields gives
     // it), so a cell the body cuts receives its n V_c / F_N particles in the
     // part outside the body; a cell the body covers stays empty
-    const double expect = (isfinite(f[0]) && f[0] > 0.f && (!p.frac || p.frac[cell] > 0.f))
-                              ? (double)f[0] * p.cell_volume / p.fnum : 0.0;
+    double expect = (isfinite(f[0]) && f[0] > 0.f && (!p.frac || p.frac[cell] > 0.f))
+                        ? (double)f[0] * p.cell_volume / p.fnum : 0.0;
+    // a cell that cannot be filled counts one more than there is room for, so
+    // that the conversion holds and the total says so
+    expect = fmin(expect, (double)p.capacity + 1.0);
     const double fl = floor(expect);
     k = (uint32_t)fl + (unit_draw(p.seed, 2 * (uint64_t)cell + 1) < expect - fl ? 1u : 0u);
     const float T = (isfinite(f[4]) && f[4] > 0.f) ? f[4] : p.temp;
@@ -96,7 +100,11 @@ __global__ void __launch_bounds__(kThreads) k_seed_cells(const SeedParams p) {
                                  (float)unit_draw(p.seed, 2 * (uint64_t)cell + 2));
     p.count[cell] = k;
   }
-  const uint32_t sum = __reduce_add_sync(0xffffffffu, k), mx = __reduce_max_sync(0xffffffffu, k);
+  // the total in 64 bits: no sum of counts may wrap round to one that fits
+  unsigned long long sum = k;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const uint32_t mx = __reduce_max_sync(0xffffffffu, k);
   if ((threadIdx.x & 31u) == 0) {
     s_sum[threadIdx.x >> 5] = sum;
     s_max[threadIdx.x >> 5] = mx;
