@@ -1103,6 +1103,7 @@ int outside_fractions(dsmc_handle* h, std::vector<float>& frac) {
 int finish_fill(dsmc_handle* h, dsmcb::InitParams& ip, uint64_t n, uint32_t* n_out) {
   ip.grid = h->grid;
   ip.cells = h->cells;
+  ip.n = (uint32_t)n;
   ip.out = soa_of(h->A);
   ip.redo = h->orig;  // dead between steps, as is the counter
   ip.n_redo = &h->meta->n_defer;

@@ -650,6 +650,23 @@ __global__ void k_cell_fields(const double* __restrict__ acc, uint32_t cells, do
 // Maxwellian.  Random numbers come from Philox (the reference used its
 // Mersenne-Twister table, which is not reproduced).
 
+// Particle k of a cell is number cell * ppc + k (ppc: the most in any cell),
+// which names its random stream.  A thread per number finds its cell by a
+// division, but numbers stop at 32 bits, and one crowded cell on a large grid
+// takes them further; WIDE: a thread per slot, its cell found among the slots
+// (cell_count is then null, as in the fills from fields), and a number's upper
+// word in the stream's next counter word.
+constexpr uint64_t kFillNumbers = 0xF0000000ull;  // leaves room for a grid's stride
+__device__ __forceinline__ uint32_t cell_of_slot(const uint32_t* slot, uint32_t cells, uint32_t d) {
+  uint32_t lo = 0, hi = cells - 1u;  // the last cell that begins at or before d: empty ones come before it
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo + 1u) / 2u;
+    if (slot[mid] <= d) lo = mid;
+    else hi = mid - 1u;
+  }
+  return lo;
+}
+
 // A position in a cell from three uniforms.
 __device__ __forceinline__ float3 fill_position(const InitParams& p, uint32_t cell, float a, float b, float c) {
   const uint32_t cx = cell % p.grid.dim.x;
@@ -667,18 +684,31 @@ __device__ __forceinline__ float3 fill_position(const InitParams& p, uint32_t ce
 // for up to 64 walks of the grid (fill of 65,536 cells around a sphere:
 // 1231 us, now 168 us in two kernels).
 constexpr uint32_t kRedraws = 64;
+template <bool WIDE>
 __global__ void __launch_bounds__(256) k_init_redraw(const __grid_constant__ InitParams p) {
   const uint32_t lane = lane_id(), n = *p.n_redo;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   // words the particle's stream has handed out before: velocity and position
   const uint32_t w0 = 4u + ((p.kind != 0 && p.cell_state && p.cell_mix) ? 1u : 0u) + 3u;
   for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
-    const uint32_t i = p.redo[r], cell = i / p.ppc, d = p.cell_slot[cell] + (i - cell * p.ppc);
+    uint32_t i, ihi = 0, cell, d;
+    if (WIDE) {
+      d = p.redo[r];
+      cell = cell_of_slot(p.cell_slot, p.cells, d);
+      const uint64_t num = (uint64_t)cell * p.ppc + (d - p.cell_slot[cell]);
+      i = (uint32_t)num;
+      ihi = (uint32_t)(num >> 32);
+    } else {
+      i = p.redo[r];
+      cell = i / p.ppc;
+      d = p.cell_slot[cell] + (i - cell * p.ppc);
+    }
     float3 q = make_float3(0.f, 0.f, 0.f);
     unsigned out = 0;
     for (uint32_t t0 = 0; t0 < kRedraws && !out; t0 += 32) {
       const uint32_t w = w0 + 3u * (t0 + lane), b = w >> 2, o = w & 3u;
-      const uint4 x = philox_block(b, i, 0u, kPurposeInit, p.seed), y = philox_block(b + 1u, i, 0u, kPurposeInit, p.seed);
+      const uint4 x = philox_block(b, i, ihi, kPurposeInit, p.seed),
+                  y = philox_block(b + 1u, i, ihi, kPurposeInit, p.seed);
       const uint32_t u[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
       auto uni = [&](uint32_t k) {
         uint32_t v = u[0];
@@ -701,15 +731,26 @@ __global__ void __launch_bounds__(256) k_init_redraw(const __grid_constant__ Ini
   }
 }
 
+template <bool WIDE>
 __global__ void k_init_fill(const __grid_constant__ InitParams p) {
-  const uint32_t total = p.cells * p.ppc;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const uint32_t cell = i / p.ppc, k = i - cell * p.ppc;
-    const uint32_t dst0 = p.cell_slot[cell];
-    if (dst0 == kNone || k >= (p.cell_count ? p.cell_count[cell] : p.cell_slot[cell + 1] - dst0)) continue;
-    const uint32_t d = dst0 + k;
+  const uint32_t total = WIDE ? p.n : p.cells * p.ppc;
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    uint32_t i, ihi = 0, cell, d;
+    if (WIDE) {
+      d = t;
+      cell = cell_of_slot(p.cell_slot, p.cells, d);
+      const uint64_t num = (uint64_t)cell * p.ppc + (d - p.cell_slot[cell]);
+      i = (uint32_t)num;
+      ihi = (uint32_t)(num >> 32);
+    } else {
+      i = t;
+      cell = i / p.ppc;
+      const uint32_t k = i - cell * p.ppc, dst0 = p.cell_slot[cell];
+      if (dst0 == kNone || k >= (p.cell_count ? p.cell_count[cell] : p.cell_slot[cell + 1] - dst0)) continue;
+      d = dst0 + k;
+    }
     PhiloxStream r;
-    r.init(p.seed, i, 0u, kPurposeInit);
+    r.init(p.seed, i, ihi, kPurposeInit);
     float3 vel;
     if (p.kind == 0) {
       const float vv = p.vmp * sqrtf(-logf(r.uniform()));
@@ -741,7 +782,7 @@ __global__ void k_init_fill(const __grid_constant__ InitParams p) {
     const float3 q = fill_position(p, cell, a, b, c);
     // a cell the mesh covers in part: a position inside the body is drawn
     // again (k_init_redraw)
-    if (p.reject_inside && inside_mesh(p.geom, q)) p.redo[atomicAdd(p.n_redo, 1u)] = i;
+    if (p.reject_inside && inside_mesh(p.geom, q)) p.redo[atomicAdd(p.n_redo, 1u)] = t;
     p.out.x[d] = q.x; p.out.y[d] = q.y; p.out.z[d] = q.z;
     p.out.u[d] = vel.x; p.out.v[d] = vel.y; p.out.w[d] = vel.z;
   }
@@ -1337,13 +1378,17 @@ cudaError_t launch_outside_fraction(const GridGeom& grid, const GeomView& geom, 
 
 cudaError_t launch_init_fill(const InitParams& p, cudaStream_t stream) {
   const uint64_t total = (uint64_t)p.cells * p.ppc;
-  const uint32_t grid = grid_for(total, 256, 8);
+  const bool wide = total > kFillNumbers;
+  if (wide && p.cell_count) return cudaErrorInvalidValue;
+  const uint32_t grid = grid_for(wide ? p.n : total, 256, 8);
   if (p.reject_inside) {
     const cudaError_t e = cudaMemsetAsync(p.n_redo, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
   }
-  k_init_fill<<<grid, 256, 0, stream>>>(p);
-  if (p.reject_inside) k_init_redraw<<<(uint32_t)num_sms() * 4u, 256, 0, stream>>>(p);
+  if (wide) k_init_fill<true><<<grid, 256, 0, stream>>>(p);
+  else k_init_fill<false><<<grid, 256, 0, stream>>>(p);
+  if (p.reject_inside && wide) k_init_redraw<true><<<(uint32_t)num_sms() * 4u, 256, 0, stream>>>(p);
+  else if (p.reject_inside) k_init_redraw<false><<<(uint32_t)num_sms() * 4u, 256, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

@@ -308,7 +308,8 @@ cudaError_t launch_seed_cells(const SeedParams& p, cudaStream_t stream);
 struct InitParams {
   GridGeom grid;
   uint32_t cells;
-  uint32_t ppc;
+  uint32_t ppc;      // most particles in a cell
+  uint32_t n;        // particles in all
   int kind;          // 0 reference sampler, 1 Maxwellian, 2 bimodal
   float vstd;        // sqrt(kT/m)
   float vstd2;       // bimodal second temperature
@@ -323,6 +324,7 @@ struct InitParams {
   int reject_inside;          // redraw positions that fall inside the mesh
   uint32_t* redo;             // with reject_inside: the particles whose first position does,
   uint32_t* n_redo;           // listed for the redraw kernel (room for all; the count zeroed)
+                              // by number, or by slot where numbers need more than 32 bits
   GeomView geom;
   const float4* cell_point;   // optional per cell: a point outside the mesh (w = 1) or none (w = 0)
   SoA out;
