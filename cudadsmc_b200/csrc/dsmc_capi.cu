@@ -45,7 +45,7 @@ struct dsmc_handle {
   bool mt_on = false;
   double* acc = nullptr;
   double* cellbuf = nullptr;  // per-cell fields / sums, cell-major, for readback (on first use)
-  unsigned char* seedbuf = nullptr;  // scratch of the fill from fields (on first use)
+  unsigned char* seedbuf = nullptr;  // scratch of the fills on sparse grids (on first use)
   Meta* meta = nullptr;
   float* inj_rem = nullptr;
   uint32_t* inj_plan = nullptr;
@@ -1076,23 +1076,68 @@ static bool geometry_in_cell(const dsmcb::GeomGrid& g, const float cmin[3], cons
 
 namespace {
 
-// Scratch of the extension fills inside the sampling accumulators (40 bytes
-// per cell, reset after the fill): per-cell Maxwellian state, an outside
-// point, the outside fraction and the free-stream share of a two-stream fill.
-float4* fill_state(dsmc_handle* h) { return reinterpret_cast<float4*>(h->acc); }
-float4* fill_point(dsmc_handle* h) { return reinterpret_cast<float4*>(h->acc) + h->cells; }
-float* fill_frac(dsmc_handle* h) { return reinterpret_cast<float*>(fill_point(h) + h->cells); }
-float* fill_mix(dsmc_handle* h) { return fill_frac(h) + h->cells; }
-static_assert(2 * sizeof(float4) + 2 * sizeof(float) <= 5 * sizeof(double),
-              "fill scratch must fit the accumulators");
+// Scratch of the extension fills: per-cell Maxwellian state, an outside point,
+// the outside fraction and the free-stream share of a two-stream fill; for a
+// fill from fields the fields, the cells' new collision state, their slots,
+// counts, scan tile sums, the scan's counters and the totals (`zero` on, to be
+// cleared).  It lies in the second state buffer, which is dead between steps,
+// so that a refused fill leaves everything as it was and a fill allocates
+// nothing; where the cells outnumber a fifth of the capacity, in a buffer of
+// the handle's own, kept from its first use on.
+struct FillScratch {
+  float4* state;
+  float4* point;
+  float* fields;
+  float2* maxrem;
+  float *frac, *mix;
+  uint32_t *slot, *count, *tile_sum;
+  Meta* meta;
+  dsmcb::SeedTotals* totals;
+  unsigned char *zero, *end;
+};
+
+int fill_scratch(dsmc_handle* h, FillScratch& f) {
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t nc = h->cells;
+  const size_t frac = up(8 * nc), mix = frac + up(4 * nc);  // behind the collision state
+  const size_t count = up(4 * (nc + 1)), tiles = count + up(4 * (nc + 1));  // behind the slots
+  const size_t meta = tiles + up(4 * (size_t)h->n_scan_tiles), totals = meta + up(sizeof(Meta));
+  const size_t part[5] = {16 * nc, 16 * nc, 20 * nc, mix + 4 * nc, totals + sizeof(dsmcb::SeedTotals)};
+  bool fits = true;
+  size_t bytes = 0;
+  for (size_t b : part) {
+    fits = fits && b <= 4 * (size_t)h->capacity;
+    bytes += up(b);
+  }
+  if (!fits && !h->seedbuf) CK(h, dalloc(&h->seedbuf, bytes), "fill scratch alloc");
+  unsigned char *at[5], *w = h->seedbuf;
+  for (int k = 0; k < 5; k++) {
+    at[k] = fits ? reinterpret_cast<unsigned char*>(h->B[k]) : w;
+    if (!fits) w += up(part[k]);
+  }
+  f.state = reinterpret_cast<float4*>(at[0]);
+  f.point = reinterpret_cast<float4*>(at[1]);
+  f.fields = reinterpret_cast<float*>(at[2]);
+  f.maxrem = reinterpret_cast<float2*>(at[3]);
+  f.frac = reinterpret_cast<float*>(at[3] + frac);
+  f.mix = reinterpret_cast<float*>(at[3] + mix);
+  f.slot = reinterpret_cast<uint32_t*>(at[4]);
+  f.count = reinterpret_cast<uint32_t*>(at[4] + count);
+  f.tile_sum = reinterpret_cast<uint32_t*>(at[4] + tiles);
+  f.meta = reinterpret_cast<Meta*>(at[4] + meta);
+  f.totals = reinterpret_cast<dsmcb::SeedTotals*>(at[4] + totals);
+  f.zero = at[4] + count;
+  f.end = at[4] + part[4];
+  return DSMC_OK;
+}
 
 // Fraction of every cell outside the mesh (all ones without one).
-int outside_fractions(dsmc_handle* h, std::vector<float>& frac) {
+int outside_fractions(dsmc_handle* h, const FillScratch& fs, std::vector<float>& frac) {
   frac.assign(h->cells, 1.f);
   if (!(h->has_geom && h->cfg.geometry)) return DSMC_OK;
   CK(h, dsmcb::launch_outside_fraction(h->grid, base_params(h, h->cfg.dt).geom, h->cells,
-                                       fill_frac(h), fill_point(h), h->stream), "outside fraction");
-  CK(h, cudaMemcpyAsync(frac.data(), fill_frac(h), h->cells * sizeof(float), cudaMemcpyDeviceToHost,
+                                       fs.frac, fs.point, h->stream), "outside fraction");
+  CK(h, cudaMemcpyAsync(frac.data(), fs.frac, h->cells * sizeof(float), cudaMemcpyDeviceToHost,
                         h->stream), "outside fraction");
   CK(h, cudaStreamSynchronize(h->stream), "outside fraction");
   return DSMC_OK;
@@ -1155,7 +1200,9 @@ int dsmc_init_state(dsmc_handle* h, const float stream_vel[3], uint32_t* n_out) 
     // of the cell outside the body, rounded stochastically from the seed;
     // positions inside the body are drawn again
     std::vector<float> frac;
-    int st = outside_fractions(h, frac);
+    FillScratch fs{};
+    int st = geo ? fill_scratch(h, fs) : DSMC_OK;
+    if (!st) st = outside_fractions(h, fs, frac);
     if (st) return st;
     const double ppc_f = c.part_per_cell ? (double)c.part_per_cell
                                          : (double)c.density * h->cell_volume / c.fnum;
@@ -1173,7 +1220,7 @@ int dsmc_init_state(dsmc_handle* h, const float stream_vel[3], uint32_t* n_out) 
     ip.reject_inside = geo;
     if (geo) {
       ip.geom = base_params(h, c.dt).geom;
-      ip.cell_point = fill_point(h);
+      ip.cell_point = fs.point;
     }
   }
   ip.kind = c.init_kind;
@@ -1204,25 +1251,20 @@ int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_
   if (two && !(c.wall_temp > 0.f)) return fail(h, DSMC_ERR_ARG, "two-stream fill needs a wall temperature");
   const bool geo = h->has_geom && c.geometry;
   const float kb_m = 1.3806e-23f / c.gas_mass;
-  // scratch of the handle: the fields, per-cell collision state, counts and
-  // slots, the scan's tile sums and counters, the totals
-  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  FillScratch fs{};
+  int st = fill_scratch(h, fs);
+  if (st) return st;
   const size_t nc = h->cells;
-  const size_t o_mr = up(5 * nc * 4), o_slot = o_mr + up(8 * nc), o_count = o_slot + up(4 * (nc + 1));
-  const size_t o_tile = o_count + up(4 * (nc + 1)), o_meta = o_tile + up(4 * (size_t)h->n_scan_tiles);
-  const size_t o_tot = o_meta + up(sizeof(Meta)), bytes = o_tot + up(sizeof(dsmcb::SeedTotals));
-  if (!h->seedbuf) CK(h, dalloc(&h->seedbuf, bytes), "seed buffer alloc");
-  unsigned char* w = h->seedbuf;
   if (geo)
-    CK(h, dsmcb::launch_outside_fraction(h->grid, base_params(h, c.dt).geom, h->cells, fill_frac(h), fill_point(h),
-                                         h->stream), "outside fraction");
-  CK(h, cudaMemcpyAsync(w, fields5, 5 * nc * sizeof(float), cudaMemcpyHostToDevice, h->stream), "seed upload");
-  CK(h, cudaMemsetAsync(w + o_count, 0, bytes - o_count, h->stream), "memset");
+    CK(h, dsmcb::launch_outside_fraction(h->grid, base_params(h, c.dt).geom, h->cells, fs.frac, fs.point, h->stream),
+       "outside fraction");
+  CK(h, cudaMemcpyAsync(fs.fields, fields5, 5 * nc * sizeof(float), cudaMemcpyHostToDevice, h->stream), "seed upload");
+  CK(h, cudaMemsetAsync(fs.zero, 0, (size_t)(fs.end - fs.zero), h->stream), "memset");
   dsmcb::SeedParams sp{};
-  sp.fields = (const float*)w;
+  sp.fields = fs.fields;
   sp.cells = h->cells;
   sp.capacity = h->capacity;
-  sp.frac = geo ? fill_frac(h) : nullptr;
+  sp.frac = geo ? fs.frac : nullptr;
   sp.cell_volume = h->cell_volume;
   sp.fnum = c.fnum;
   sp.temp = c.temp;
@@ -1232,15 +1274,15 @@ int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_
   sp.weight = weight;
   for (int q = 0; q < 3; q++) sp.stream[q] = c.stream_vel[q];
   sp.seed = c.seed ^ 0x2545F4914F6CDD1Dull;
-  sp.state = fill_state(h);
-  sp.share = two ? fill_mix(h) : nullptr;
-  sp.maxrem = (float2*)(w + o_mr);
-  sp.count = (uint32_t*)(w + o_count);
-  sp.tile_sum = (uint32_t*)(w + o_tile);
-  sp.totals = (dsmcb::SeedTotals*)(w + o_tot);
+  sp.state = fs.state;
+  sp.share = two ? fs.mix : nullptr;
+  sp.maxrem = fs.maxrem;
+  sp.count = fs.count;
+  sp.tile_sum = fs.tile_sum;
+  sp.totals = fs.totals;
   CK(h, dsmcb::launch_seed_cells(sp, h->stream), "seed cells");
-  CK(h, dsmcb::launch_scan(sp.count, nullptr, (uint32_t*)(w + o_slot), h->cells, sp.tile_sum, h->n_scan_tiles,
-                           (Meta*)(w + o_meta), 0, h->stream), "seed scan");
+  CK(h, dsmcb::launch_scan(sp.count, nullptr, fs.slot, h->cells, sp.tile_sum, h->n_scan_tiles, fs.meta, 0,
+                           h->stream), "seed scan");
   dsmcb::SeedTotals tot{};
   CK(h, cudaMemcpyAsync(&tot, sp.totals, sizeof(tot), cudaMemcpyDeviceToHost, h->stream), "seed totals");
   CK(h, cudaStreamSynchronize(h->stream), "seed totals");
@@ -1253,18 +1295,18 @@ int seed_from_fields(dsmc_handle* h, const float* fields5, float weight, uint32_
   ip.ppc = kmax;
   ip.kind = DSMC_INIT_MAXWELL;
   ip.seed = make_uint2((uint32_t)c.seed, (uint32_t)(c.seed >> 32));
-  ip.cell_state = fill_state(h);
+  ip.cell_state = fs.state;
   if (two) {
-    ip.cell_mix = fill_mix(h);
+    ip.cell_mix = fs.mix;
     ip.stream = make_float3(c.stream_vel[0], c.stream_vel[1], c.stream_vel[2]);
     ip.vstd = std::sqrt(kb_m * c.temp);
   }
   ip.reject_inside = geo;
   if (geo) {
     ip.geom = base_params(h, c.dt).geom;
-    ip.cell_point = fill_point(h);
+    ip.cell_point = fs.point;
   }
-  ip.cell_slot = (const uint32_t*)(w + o_slot);
+  ip.cell_slot = fs.slot;
   return finish_fill(h, ip, n, n_out);
 }
 
