@@ -126,6 +126,44 @@ struct __align__(128) Smem {
 __device__ __forceinline__ int chunk128(int r, int c) { return 128 * r + 16 * (c ^ (r & 7)); }
 __device__ __forceinline__ int chunk64(int r, int c) { return 64 * r + 16 * (c ^ ((r >> 1) & 3)); }
 
+// A staged block out by plain stores, a row's 32 columns at a time: where the
+// rows are not 16-byte aligned, and where C is read back (beta) or added to
+// (splits).  Each lane storing its own row touched 32 rows at once (1 x 327680
+// x 256 with beta 288 us, split four ways 426; now 82 and 191).  The rows' loads
+// of C are in flight together; beta's sums go back to the block.
+__device__ __forceinline__ void rows_out(const GemmArgs& g, unsigned char* blk, int row0, int c0) {
+  const int lane = threadIdx.x & 31, rows = min(32, g.m - row0);
+  if (c0 + lane >= g.n) return;
+  float* cp = g.c + (size_t)row0 * g.ldc + c0 + lane;
+  const bool back = g.beta != 0.f && g.splits == 1;
+  float old[32];
+#pragma unroll
+  for (int r = 0; r < 32; r++) old[r] = back && r < rows ? cp[(size_t)r * g.ldc] : 0.f;
+#pragma unroll
+  for (int r = 0; r < 32; r++) {
+    if (r >= rows) break;
+    float* at = reinterpret_cast<float*>(blk + chunk128(r, lane >> 2) + 4 * (lane & 3));
+    float x = *at;
+    if (g.splits > 1) {
+      atomicAdd(cp + (size_t)r * g.ldc, x);
+    } else {
+      if (back) {
+        x += g.beta * old[r];
+        *at = x;
+      }
+      cp[(size_t)r * g.ldc] = x;
+    }
+  }
+}
+__device__ __forceinline__ void rows_out_bf16(const GemmArgs& g, const unsigned char* blk, int row0, int c0) {
+  const int lane = threadIdx.x & 31, rows = min(32, g.m - row0);
+  if (c0 + lane >= g.n) return;
+  bf16* cp = g.cb + (size_t)row0 * g.ldcb + c0 + lane;
+#pragma unroll 8
+  for (int r = 0; r < rows; r++)
+    cp[(size_t)r * g.ldcb] = *reinterpret_cast<const bf16*>(blk + chunk64(r, lane >> 3) + 2 * (lane & 7));
+}
+
 // The tiles of CTA `b` of `g`.  Plain: all (m, n, split) items round robin, m
 // fastest, so that the tiles that share a column block of B run side by side
 // and B comes from memory once.  COLS: whole columns of tiles, m innermost,
@@ -420,22 +458,24 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
         // this warp's staging buffers are free again
         if (lane == 0) bulk_wait_read<Sh::kStaging - 1>();
         __syncwarp();
-        if (g.tma_c) {
+        if (MSE && !g.tma_c) {  // (a field off 16 bytes; as rows_out the kernel spills twice as much)
+#pragma unroll
+          for (int i = 0; i < 32; i++)
+            if (row < g.m && c0 + i < g.n) g.c[(size_t)row * g.ldc + c0 + i] = v[i];
+        } else if (g.c) {
 #pragma unroll
           for (int i = 0; i < 8; i++)
             *reinterpret_cast<float4*>(fst + 4096 * buf + chunk128(lane, i)) =
                 make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        } else if (g.c) {
-          if (row < g.m) {
+          if (!MSE && !g.tma_c) {
+            __syncwarp();
+            rows_out(g, fst + 4096 * buf, row0, c0);
+            __syncwarp();
+            if (g.beta != 0.f) {  // the sum, for the BF16 copy
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-              if (c0 + i >= g.n) continue;
-              float* cp = &g.c[(size_t)row * g.ldc + c0 + i];
-              if (g.splits > 1) {
-                atomicAdd(cp, v[i]);
-              } else {
-                if (g.beta != 0.f) v[i] += g.beta * *cp;
-                *cp = v[i];
+              for (int i = 0; i < 8; i++) {
+                const float4 x = *reinterpret_cast<const float4*>(fst + 4096 * buf + chunk128(lane, i));
+                v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
               }
             }
           }
@@ -501,15 +541,20 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
             const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
             p[i] = *reinterpret_cast<const uint32_t*>(&b);
           }
-          if (g.tma_cb) {
+          if (MSE && !g.tma_cb) {
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+              if (row < g.m && c0 + i < g.n) g.cb[(size_t)row * g.ldcb + c0 + i] = __float2bfloat16(v[i]);
+          } else {
 #pragma unroll
             for (int i = 0; i < 4; i++)
               *reinterpret_cast<uint4*>(hst + 2048 * buf + chunk64(lane, i)) =
                   make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
-          } else if (row < g.m) {
-#pragma unroll
-            for (int i = 0; i < 32; i++)
-              if (c0 + i < g.n) g.cb[(size_t)row * g.ldcb + c0 + i] = __float2bfloat16(v[i]);
+          }
+          if (!MSE && !g.tma_cb) {
+            __syncwarp();
+            rows_out_bf16(g, hst + 2048 * buf, row0, c0);
+            __syncwarp();
           }
         }
         if constexpr (MSE) {
