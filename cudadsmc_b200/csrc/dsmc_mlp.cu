@@ -68,6 +68,18 @@ __global__ void __launch_bounds__(32 * kColWarps) k_colsum(const float* x, int r
   dsmcb::beside_exit(beside);
 }
 
+// The same sums, a thread per column straight from memory: few rows, or so
+// many columns that they fill the GPU by themselves (the staged form's blocks
+// then come in many waves: 16 x 327680 37 us, here 5; 128 x 81920 15 and 8; but
+// 128 x 8192 5 and 7, 1024 x 81920 65 and 80).
+__global__ void k_colsum_wide(const float* x, int rows, int cols, int ld, float* out) {
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  if (col >= cols) return;
+  float s = 0.f;
+  for (int r = 0; r < rows; r++) s += x[(size_t)r * ld + col];
+  out[col] = s;
+}
+
 // Masked MSE: targets that are NaN carry no loss.  dy = scale * 2 (y - t).
 __global__ void k_mse_grad(const float* y, const bf16* t, size_t n, float scale, bf16* dyb, float* dy,
                            double* loss, unsigned long long* count) {
@@ -189,7 +201,11 @@ int dsmc_gelu_backward(const float* z, const float* dh, float* dz, void* dz_bf16
 
 int dsmc_colsum(const float* x, int rows, int cols, int ld, float* out, void* stream) {
   if (!x || !out || rows < 0 || cols <= 0) return DSMC_ERR_ARG;
-  k_colsum<<<(cols + 31) / 32, 32 * kColWarps, 0, (cudaStream_t)stream>>>(x, rows, cols, ld, out, false);
+  // measured between 1 and 1024 rows of 512 to 327,680 columns: the forms meet
+  // at about one row per 150 columns
+  cudaStream_t s = (cudaStream_t)stream;
+  if (rows <= 16 || (int64_t)rows * 150 <= cols) k_colsum_wide<<<(cols + 255) / 256, 256, 0, s>>>(x, rows, cols, ld, out);
+  else k_colsum<<<(cols + 31) / 32, 32 * kColWarps, 0, s>>>(x, rows, cols, ld, out, false);
   return cudaGetLastError() == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
 }
 
