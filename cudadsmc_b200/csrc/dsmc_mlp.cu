@@ -165,8 +165,13 @@ __global__ void __launch_bounds__(256) k_adam(float* w, const float* g, float* m
     }
   }
   for (size_t i = done + t0; i < n; i += nt) {
-    adam_one(a, g[i], w[i], m[i], v[i]);
-    if (wb) wb[i] = __float2bfloat16(w[i]);
+    const float gi = g[i];  // all four loads before the first store
+    float wi = w[i], mi = m[i], vi = v[i];
+    adam_one(a, gi, wi, mi, vi);
+    m[i] = mi;
+    v[i] = vi;
+    w[i] = wi;
+    if (wb) wb[i] = __float2bfloat16(wi);
   }
   dsmcb::beside_exit(beside);
 }
