@@ -352,6 +352,7 @@ struct ScatterOut {
   __device__ __forceinline__ uint2 get(uint32_t d) const {
     return PAIR ? reinterpret_cast<const uint2*>(val)[d] : make_uint2(val[d], pos[d]);
   }
+  __device__ __forceinline__ uint32_t position(uint32_t d) const { return PAIR ? val[2 * (size_t)d + 1] : pos[d]; }
 };
 
 template <bool PAIR>
@@ -399,14 +400,58 @@ __global__ void __launch_bounds__(256) k_scatter_kv(const uint32_t* __restrict__
 // few thousand keys reach every SM (4,096 keys of 24: 35 us with tiles of 256
 // keys on 16 CTAs, now 5 us; 524,288 keys of 8: 58, now 34 us).
 constexpr int kFixupThreads = 128, kFixupCap = 1024;
+
+// Keys with more than kLargeKey entries are ranked by themselves: entries
+// [i0, i0 + Q kFixupThreads) of such a key, m at s0 (the whole CTA).  Each
+// thread ranks Q of them against the key's positions, kFixupCap at a time in
+// shared memory, four per load.  Bound by the comparisons, m squared of them:
+// 4.2M entries of which 1 % are in keys of 2,500, 524,288 keys: 4.2 ms with
+// chunks of 4,096 entries and 256 threads, 4.4 with chunks of 1,024 and larger
+// keys ranked from global memory, now 1.9; 256 keys of 16,384 4.7 s -> 53 ms.
+constexpr uint32_t kLargeKey = 256;
+template <int Q, bool PAIR>
+__device__ __forceinline__ void rank_large_key(uint32_t* spos, const ScatterOut<PAIR>& in, uint32_t s0, uint32_t m,
+                                               uint32_t i0, uint32_t key, uint32_t* keys_out, uint32_t* vals_out) {
+  uint32_t my[Q], val[Q], rank[Q];
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    const uint32_t t = i0 + threadIdx.x + q * kFixupThreads;
+    const uint2 e = t < m ? in.get(s0 + t) : make_uint2(0u, 0u);
+    val[q] = e.x;
+    my[q] = e.y;
+    rank[q] = 0;
+  }
+  for (uint32_t j0 = 0; j0 < m; j0 += kFixupCap) {
+    const uint32_t nj = min((uint32_t)kFixupCap, m - j0);
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < kFixupCap; t += kFixupThreads)
+      spos[t] = t < nj ? in.position(s0 + j0 + t) : kNone;  // (counts for nobody)
+    __syncthreads();
+#pragma unroll 2
+    for (uint32_t j = 0; j < nj; j += 4) {
+      const uint4 o = *reinterpret_cast<const uint4*>(spos + j);
+#pragma unroll
+      for (int q = 0; q < Q; q++)
+        rank[q] += (uint32_t)(o.x < my[q]) + (uint32_t)(o.y < my[q]) + (uint32_t)(o.z < my[q]) + (uint32_t)(o.w < my[q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    if (i0 + threadIdx.x + q * kFixupThreads >= m) break;
+    keys_out[s0 + rank[q]] = key;
+    vals_out[s0 + rank[q]] = val[q];
+  }
+}
+
 template <bool PAIR>
 __global__ void __launch_bounds__(kFixupThreads) k_segment_fixup(const uint32_t* __restrict__ start, uint32_t nkeys,
                                                                  uint32_t kt, ScatterOut<PAIR> in,
                                                                  uint32_t* __restrict__ keys_out,
                                                                  uint32_t* __restrict__ vals_out) {
   __shared__ uint32_t ls[kFixupThreads + 1];
-  __shared__ uint32_t spos[kFixupCap];
+  __shared__ __align__(16) uint32_t spos[kFixupCap];
   __shared__ uint8_t cellof[kFixupCap];  // the chunk's key of each entry
+  __shared__ uint32_t first;
   const uint32_t ntiles = (nkeys + kt - 1) / kt;
   for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint32_t c0 = tile * kt, nct = min(kt, nkeys - c0);
@@ -418,16 +463,28 @@ __global__ void __launch_bounds__(kFixupThreads) k_segment_fixup(const uint32_t*
       const uint32_t base = ls[cur];
       const uint32_t c = cur + 1 + threadIdx.x;
       const int fits = (c <= nct) && (ls[c] - base <= (uint32_t)kFixupCap);
-      const uint32_t k = __syncthreads_count(fits);
+      uint32_t k = __syncthreads_count(fits);
+      // a chunk ends before a large key
+      const bool large = threadIdx.x <= k && c <= nct && ls[c] - ls[c - 1] > kLargeKey;
+      if (__syncthreads_or(large)) {
+        if (threadIdx.x == 0) first = k;
+        __syncthreads();
+        if (large) atomicMin(&first, threadIdx.x);
+        __syncthreads();
+        k = first;
+      }
       if (k == 0) {
-        // one key with more than kFixupCap entries: rank from global memory
-        const uint32_t s0 = base, e0 = ls[cur + 1];
-        for (uint32_t i = s0 + threadIdx.x; i < e0; i += blockDim.x) {
-          const uint2 my = in.get(i);
-          uint32_t rank = 0;
-          for (uint32_t j = s0; j < e0; j++) rank += in.get(j).y < my.y;
-          keys_out[s0 + rank] = c0 + cur;
-          vals_out[s0 + rank] = my.x;
+        // one large key, in passes of nearly equal size
+        const uint32_t m = ls[cur + 1] - base, key = c0 + cur;
+        const uint32_t passes = (m + kFixupCap - 1) / kFixupCap;
+        const uint32_t q = (m + passes * kFixupThreads - 1) / (passes * kFixupThreads);  // entries per thread
+        for (uint32_t i0 = 0; i0 < m; i0 += q * kFixupThreads) {
+          if (q <= 3) rank_large_key<3>(spos, in, base, m, i0, key, keys_out, vals_out);
+          else if (q == 4) rank_large_key<4>(spos, in, base, m, i0, key, keys_out, vals_out);
+          else if (q == 5) rank_large_key<5>(spos, in, base, m, i0, key, keys_out, vals_out);
+          else if (q == 6) rank_large_key<6>(spos, in, base, m, i0, key, keys_out, vals_out);
+          else if (q == 7) rank_large_key<7>(spos, in, base, m, i0, key, keys_out, vals_out);
+          else rank_large_key<8>(spos, in, base, m, i0, key, keys_out, vals_out);
         }
         cur += 1;
         __syncthreads();
