@@ -525,47 +525,44 @@ __global__ void __launch_bounds__(kFixupThreads) k_segment_fixup(const uint32_t*
 
 // FindCellBoundariesDev (kernels/dsmc_kernel.cu:1734-1787): start/end per
 // cell from sorted keys (cse zeroed by the caller) and the gather.
-// Each thread gathers four particles at a time, their 24 loads in flight
-// together (4.2M particles: 66 -> 61 us, 3.8 TB/s: what is left is the gather's
-// sectors and the bounds' scattered words).
+// A particle's six loads are in flight together, before its stores, and a
+// thread takes one at a time: four gather slower (4.2M particles moved by less
+// than 50 places: 74 us with a load and a store after the other, 53 with four
+// particles' 24 loads, now 45).  The bounds alone are taken four at a time
+// (20M keys: 33 us one at a time), in a kernel without the gather's registers.
+template <bool GATHER>
 __global__ void __launch_bounds__(256) k_bounds_reorder(const uint32_t* __restrict__ keys,
                                                         const uint32_t* __restrict__ idx, uint32_t n, uint32_t ncells,
-                                                        uint2* cse, SoA src, SoA dst, int gather) {
-  constexpr int U = 4;
+                                                        uint2* cse, SoA src, SoA dst) {
+  constexpr int U = GATHER ? 1 : 4;
   for (uint32_t base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
-    uint32_t s[U];
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      const uint32_t i = base + k * blockDim.x + threadIdx.x;
-      s[k] = gather && i < n ? idx[i] : 0u;
+    uint32_t h[U], hp[U];
+    float v[6];
+    const uint32_t i0 = base + threadIdx.x;
+    if (GATHER && i0 < n) {
+      const uint32_t s = idx[i0];
+      v[0] = src.x[s]; v[1] = src.y[s]; v[2] = src.z[s];
+      v[3] = src.u[s]; v[4] = src.v[s]; v[5] = src.w[s];
     }
 #pragma unroll
     for (int k = 0; k < U; k++) {
-      const uint32_t i = base + k * blockDim.x + threadIdx.x;
+      const uint32_t i = i0 + k * blockDim.x;
+      h[k] = i < n ? keys[i] : kNone;
+      hp[k] = i > 0 && i < n ? keys[i - 1] : kNone;
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const uint32_t i = i0 + k * blockDim.x;
       if (i >= n) continue;
-      const uint32_t h = keys[i];
-      const uint32_t hp = i > 0 ? keys[i - 1] : kNone;
-      if (i == 0 || h != hp) {
-        if (h < ncells) cse[h].x = i;
-        if (i > 0 && hp < ncells) cse[hp].y = i;
+      if (i == 0 || h[k] != hp[k]) {
+        if (h[k] < ncells) cse[h[k]].x = i;
+        if (i > 0 && hp[k] < ncells) cse[hp[k]].y = i;
       }
-      if (i == n - 1 && h < ncells) cse[h].y = i + 1;
+      if (i == n - 1 && h[k] < ncells) cse[h[k]].y = i + 1;
     }
-    if (!gather) continue;
-    float v[6][U];
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      const uint32_t i = base + k * blockDim.x + threadIdx.x;
-      if (i >= n) continue;
-      v[0][k] = src.x[s[k]]; v[1][k] = src.y[s[k]]; v[2][k] = src.z[s[k]];
-      v[3][k] = src.u[s[k]]; v[4][k] = src.v[s[k]]; v[5][k] = src.w[s[k]];
-    }
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      const uint32_t i = base + k * blockDim.x + threadIdx.x;
-      if (i >= n) continue;
-      dst.x[i] = v[0][k]; dst.y[i] = v[1][k]; dst.z[i] = v[2][k];
-      dst.u[i] = v[3][k]; dst.v[i] = v[4][k]; dst.w[i] = v[5][k];
+    if (GATHER && i0 < n) {
+      dst.x[i0] = v[0]; dst.y[i0] = v[1]; dst.z[i0] = v[2];
+      dst.u[i0] = v[3]; dst.v[i0] = v[4]; dst.w[i0] = v[5];
     }
   }
 }
@@ -1072,9 +1069,10 @@ cudaError_t launch_bounds_reorder(const uint32_t* keys, const uint32_t* idx, uin
         const_cast<float*>(src ? src[4] : nullptr), const_cast<float*>(src ? src[5] : nullptr)};
   SoA d{dst ? dst[0] : nullptr, dst ? dst[1] : nullptr, dst ? dst[2] : nullptr,
         dst ? dst[3] : nullptr, dst ? dst[4] : nullptr, dst ? dst[5] : nullptr};
-  const uint32_t grid = grid_for(n, 1024, 8);
-  k_bounds_reorder<<<grid, 256, 0, stream>>>(keys, idx, n, ncells, (uint2*)cse, s, d,
-                                             (src && dst) ? 1 : 0);
+  if (src && dst)
+    k_bounds_reorder<true><<<grid_for(n, 256, 8), 256, 0, stream>>>(keys, idx, n, ncells, (uint2*)cse, s, d);
+  else
+    k_bounds_reorder<false><<<grid_for(n, 1024, 8), 256, 0, stream>>>(keys, idx, n, ncells, (uint2*)cse, s, d);
   return cudaGetLastError();
 }
 
