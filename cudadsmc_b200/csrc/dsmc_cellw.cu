@@ -535,18 +535,27 @@ constexpr uint32_t kNtcClaim = 256;  // claim slots per warp: the largest chunk
 // memory and its random words come a block at a time (64x32x32 sphere flow,
 // 27 -> 19 us with the claims).  The two-CTA register cap keeps it free of
 // spills: 3 CTAs ran the sphere flow's 3 us slower, the capsule's 1 us faster.
-template <int WARPS>
+template <int WARPS, int RNG, bool STAGED>
 __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb, const uint32_t vg) {
-  __shared__ uint32_t s_claim[WARPS][kNtcClaim];
-  __shared__ float s_vel[WARPS][3][kNtcClaim];
+  constexpr bool kDense = RNG != 0;  // the reference's streams have no dense cells
+  __shared__ uint32_t s_claim[kDense ? WARPS : 1][kDense ? kNtcClaim : 1];
+  constexpr bool kStaged = kDense && STAGED;
+  __shared__ float s_vel[kStaged ? WARPS : 1][3][kStaged ? kNtcClaim : 1];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t step = p.step_override ? p.step_override : p.meta->step;
-  const bool taus = p.rng_kind == 0;
-  for (uint32_t t = lane; t < kNtcClaim; t += 32) s_claim[warp][t] = 0xffffffffu;
-  __syncwarp();
+  const bool taus = RNG < 0 ? p.rng_kind == 0 : RNG == 0;
+  if constexpr (kDense) {
+    for (uint32_t t = lane; t < kNtcClaim; t += 32) s_claim[warp][t] = 0xffffffffu;
+    __syncwarp();
+  }
   uint32_t col = 0;
   double sum_g = 0.0;
-  const uint32_t nl = p.meta->n_light, nh1 = p.meta->n_heaviest, nh = nh1 + p.meta->n_heavy;
+  const uint32_t nl = p.meta->n_light;
+  uint32_t nh1 = 0, nh = 0;
+  if constexpr (kDense) {
+    nh1 = p.meta->n_heaviest;
+    nh = nh1 + p.meta->n_heavy;
+  }
   const uint32_t gw = vb * WARPS + warp, nw = vg * WARPS;
   const uint32_t nlw = nw > nh ? nw - nh : 0u;  // warps without a dense cell
   // few cells: one item per warp and no claims, the light cells spread over
@@ -563,15 +572,15 @@ __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb,
     const bool ahead = it >= nh1;
     uint32_t next = items;
     if (!once && ahead && lane == 0) next = nw + atomicAdd(claims, 1u);
-    if (it < nh) {
+    if (kDense && it < nh) {
       const uint4 e = p.ntc_heavy[it < nh1 ? it : p.cells - 1u - (it - nh1)];
       // the cell's velocities in shared memory for the selections: its rounds
       // are one warp's chain, and every particle is touched several times
-      float* su = s_vel[warp][0];
-      float* sv = s_vel[warp][1];
-      float* sw = s_vel[warp][2];
+      float* su = s_vel[kStaged ? warp : 0u][0];
+      float* sv = s_vel[kStaged ? warp : 0u][1];
+      float* sw = s_vel[kStaged ? warp : 0u][2];
       // (but for a cell above the chunk that does not fit)
-      const bool fits = e.z <= kNtcClaim;
+      const bool fits = kStaged && e.z <= kNtcClaim;
       for (uint32_t t = lane; fits && t < e.z; t += 32) {
         su[t] = p.mid.u[e.y + t];
         sv[t] = p.mid.v[e.y + t];
@@ -585,7 +594,7 @@ __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb,
         vmax = ntc_select_fast_warp(p, e.x, e.z, acc, reinterpret_cast<float*>(s_claim[warp]), step, e.w & ~kGiantPairs, vm.x, col, sum_g);
         for (uint32_t t = lane; t < 128u; t += 32) s_claim[warp][t] = 0xffffffffu;
       } else {
-        const GlobalVel acc{su, sv, sw, 0u};
+        const GlobalVel acc = kStaged ? GlobalVel{su, sv, sw, 0u} : GlobalVel{p.mid.u, p.mid.v, p.mid.w, e.y};
         vmax = ntc_select_heavy_warp(p, e.x, e.z, acc, s_claim[warp], step, e.w, vm.x, col, sum_g);
       }
       __syncwarp();
@@ -625,10 +634,12 @@ __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb,
   }
 }
 
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 2) k_ntc_w(const __grid_constant__ StepParams p) {
+// RNG: the random streams of the kernel (StepParams::rng_kind), -1: by p.
+// STAGED: dense cells' velocities in shared memory, else in place.
+template <int WARPS, int RNG, int MINB, bool STAGED>
+__global__ void __launch_bounds__(WARPS * 32, MINB) k_ntc_w(const __grid_constant__ StepParams p) {
   chained_entry();
-  ntc_body<WARPS>(p, blockIdx.x, gridDim.x);
+  ntc_body<WARPS, RNG, STAGED>(p, blockIdx.x, gridDim.x);
 }
 // The NTC kernel's share of a batched grid: one block per member and the rest
 // by the members' listed work (32 light cells or one dense cell each take a
@@ -675,7 +686,7 @@ template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 5) k_ntc_wb(const __grid_constant__ BatchOf<StepParams> bv) {
   chained_entry();
   uint32_t member, vb, vg;
-  if (ntc_share(bv, member, vb, vg)) ntc_body<WARPS>(bv.items[member], vb, vg);
+  if (ntc_share(bv, member, vb, vg)) ntc_body<WARPS, -1, true>(bv.items[member], vb, vg);
 }
 
 // ------------------------------------------------ flight + keys + sample ----
@@ -1311,7 +1322,8 @@ cudaError_t launch_flight_pw(const StepParams& p, cudaStream_t stream) {
 constexpr int kNtcWarps = 8;
 constexpr int kNtcWarpsB = 4;  // batched: 20 warps per SM without spills
 
-cudaError_t launch_ntc_w(const StepParams& p, cudaStream_t stream) {
+template <int WARPS, int RNG, int MINB, bool STAGED>
+cudaError_t launch_ntc_shape(const StepParams& p, cudaStream_t stream) {
   static LaunchShapeW cache[8];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1319,13 +1331,32 @@ cudaError_t launch_ntc_w(const StepParams& p, cudaStream_t stream) {
   LaunchShapeW& ls = cache[dev & 7];
   if (ls.device != dev) {
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ntc_w<kNtcWarps>, kNtcWarps * 32, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ntc_w<WARPS, RNG, MINB, STAGED>, WARPS * 32, 0);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     ls.device = dev;
     ls.per_sm = per_sm;
   }
-  return launch_chained(k_ntc_w<kNtcWarps>, (uint32_t)(num_sms() * ls.per_sm), kNtcWarps * 32, 0, stream, Chain(true, p.carveout), p);
+  return launch_chained(k_ntc_w<WARPS, RNG, MINB, STAGED>, (uint32_t)(num_sms() * ls.per_sm), WARPS * 32, 0, stream,
+                        Chain(true, p.carveout), p);
+}
+cudaError_t launch_ntc_w(const StepParams& p, cudaStream_t stream) {
+  // Reference streams: light cells only, so 72 registers and 3 CTAs (a form
+  // for both kinds of stream takes 104 and 2).  12.8M particles, 1.6M cells:
+  // step 774 -> 735 us; 524,288 of 8 249 -> 237; 16^3 cells of 24 48.5 -> 44.1.
+  if (p.rng_kind == 0) return launch_ntc_shape<kNtcWarps, 0, 3, false>(p, stream);
+  // Philox: 16 warps per SM, or 20 in smaller CTAs where the light cells are
+  // many times the lanes (1.6M cells of 8: 108 -> 100 us, 524,288 of 8 42.2 ->
+  // 39.9, 196,608 of 8 21.9 -> 21.3), but not for fewer cells (147,456 of 8: 18.6
+  // -> 19.4) or more particles per cell (524,288 of 16: 67.1 -> 70.8, of 12
+  // 54.4 -> 52.3).  Where dense cells are many times the warps, what counts is
+  // how many are under way, not each one's chain: 24 warps, velocities in
+  // place (524,288 cells of 30: 388 -> 316 us, of 24 151 -> 137; 110,592 of 20 32.7
+  // -> 39.4, a sphere flow of 524,288 of 21 59.5 -> 64.5).
+  const float lanes = (float)num_sms() * 16.f * 32.f, cells = (float)p.cells;
+  if (cells >= 5.f * lanes && p.avg_conc >= 24.f) return launch_ntc_shape<kNtcWarps, 1, 3, false>(p, stream);
+  if (cells >= 2.5f * lanes && p.avg_conc < 14.f) return launch_ntc_shape<4, 1, 5, true>(p, stream);
+  return launch_ntc_shape<kNtcWarps, 1, 2, true>(p, stream);
 }
 
 template <int MINB, bool COOP>
