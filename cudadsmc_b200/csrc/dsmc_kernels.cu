@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(32 * kCollideWarps) k_collide_cells(const __gr
       CellState st{p.maxrem + hc, nullptr, p.stat4 ? p.stat4 + hc : nullptr};
       GlobalVel acc{p.in.u, p.in.v, p.in.w, hs};
       if (hn > kCollideClaim) {
-        ntc_heavy_warp(p, hc, hn, acc, nullptr, p.step_override, st, sel, col, sum_g);
+        ntc_heavy_warp<false>(p, hc, hn, acc, nullptr, p.step_override, st, sel, col, sum_g);
       } else {
         float* su = s_vel[warp][0];
         float* sv = s_vel[warp][1];

@@ -374,8 +374,8 @@ __device__ __forceinline__ void collide_cell(const StepParams& p, uint32_t cell,
 // same pair.  Acceptance uses (sigma*g)max as of the round's start.  M pairs
 // from vmax_in; returns the new (sigma*g)max (the same in every lane).
 // claim[] holds 0xffffffff for every claim index of the cell and is left so;
-// without one (null) the lanes compare their pairs with the lower lanes'.
-template <class Acc>
+// without it (CLAIM false) the lanes compare their pairs with the lower lanes'.
+template <bool CLAIM = true, class Acc>
 __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint32_t cell,
                                                        uint32_t n, Acc acc, uint32_t* claim,
                                                        uint32_t step, uint32_t M, float vmax_in,
@@ -400,7 +400,7 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
     drawn += want;
     uint32_t ji = 0, jj = 0;
     bool win = pend;
-    if (claim) {
+    if (CLAIM) {
       if (pend) {
         ji = acc.claim_index(pi);
         jj = acc.claim_index(pj);
@@ -432,7 +432,7 @@ __device__ __forceinline__ float ntc_select_heavy_warp(const StepParams& p, uint
       }
     }
     __syncwarp();
-    if (claim && pend) {
+    if (CLAIM && pend) {
       claim[ji] = 0xffffffffu;
       claim[jj] = 0xffffffffu;
     }
@@ -522,7 +522,7 @@ __device__ __forceinline__ float ntc_select_fast_warp(const StepParams& p, uint3
   return vmax;
 }
 
-template <class Acc>
+template <bool CLAIM = true, class Acc>
 __device__ __forceinline__ void ntc_heavy_warp(const StepParams& p, uint32_t cell, uint32_t n,
                                                Acc acc, uint32_t* claim, uint32_t step,
                                                CellState cs, uint32_t& sel, uint32_t& col,
@@ -532,7 +532,7 @@ __device__ __forceinline__ void ntc_heavy_warp(const StepParams& p, uint32_t cel
   const float fpc = ntc_fpc_fast(p, n, vm);
   const uint32_t M = (uint32_t)fpc;
   const uint32_t col0 = col;
-  const float vmax = ntc_select_heavy_warp(p, cell, n, acc, claim, step, M, vm.x, col, sum_g);
+  const float vmax = ntc_select_heavy_warp<CLAIM>(p, cell, n, acc, claim, step, M, vm.x, col, sum_g);
   const uint32_t wcol = warp_sum(col - col0);
   if (lane == 0) {
     sel += M;
