@@ -1165,6 +1165,28 @@ int finish_fill(dsmc_handle* h, dsmcb::InitParams& ip, uint64_t n, uint32_t* n_o
   return DSMC_OK;
 }
 
+// InitSystemState / GenerateInitialVelocities (kernels/dsmc_kernel.cu:394-427):
+// ppc = floor(n V_c / F_N) particles in every cell the mesh does not touch.
+// Returns their number.
+uint64_t reference_slots(const dsmc_handle* h, bool geo, std::vector<uint32_t>& slot, std::vector<uint32_t>& count) {
+  const dsmc_config& c = h->cfg;
+  uint64_t n = 0;
+  for (uint32_t cell = 0; cell < h->cells; cell++) {
+    uint32_t cx = cell % c.grid_dim[0], cy = (cell / c.grid_dim[0]) % c.grid_dim[1],
+             cz = cell / (c.grid_dim[0] * c.grid_dim[1]);
+    float cmin[3] = {c.grid_min[0] + cx * h->cell_size[0], c.grid_min[1] + cy * h->cell_size[1],
+                     c.grid_min[2] + cz * h->cell_size[2]};
+    if (geo && geometry_in_cell(h->ggrid, cmin, h->cell_size)) {
+      slot[cell] = 0xffffffffu;
+      continue;
+    }
+    slot[cell] = (uint32_t)n;
+    count[cell] = h->ppc;
+    n += h->ppc;
+  }
+  return n;
+}
+
 double unit_draw(uint64_t& mix) { return (double)(splitmix64(mix) >> 11) / 9007199254740992.0; }
 
 }  // namespace
@@ -1179,21 +1201,7 @@ int dsmc_init_state(dsmc_handle* h, const float stream_vel[3], uint32_t* n_out) 
   dsmcb::InitParams ip{};
   uint64_t mix = c.seed ^ 0x5DEECE66Dull;
   if (reference) {
-    // InitSystemState / GenerateInitialVelocities (kernels/dsmc_kernel.cu:394-427):
-    // ppc = floor(n V_c / F_N) particles in every cell the mesh does not touch
-    for (uint32_t cell = 0; cell < h->cells; cell++) {
-      uint32_t cx = cell % c.grid_dim[0], cy = (cell / c.grid_dim[0]) % c.grid_dim[1],
-               cz = cell / (c.grid_dim[0] * c.grid_dim[1]);
-      float cmin[3] = {c.grid_min[0] + cx * h->cell_size[0], c.grid_min[1] + cy * h->cell_size[1],
-                       c.grid_min[2] + cz * h->cell_size[2]};
-      if (geo && geometry_in_cell(h->ggrid, cmin, h->cell_size)) {
-        slot[cell] = 0xffffffffu;
-        continue;
-      }
-      slot[cell] = (uint32_t)n;
-      count[cell] = h->ppc;
-      n += h->ppc;
-    }
+    n = reference_slots(h, geo, slot, count);
     ip.ppc = h->ppc;
   } else {
     // the Maxwellian and bimodal starts: n V_c / F_N particles times the part
