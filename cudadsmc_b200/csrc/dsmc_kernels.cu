@@ -19,11 +19,13 @@ namespace {
 using namespace dev;
 
 // Move stage: free flight and boundaries for n particles in place.  Without a
-// body each thread flies four at a time, their loads in flight together (4.2M
-// particles: 50 -> 28 us).
-template <bool BODY>
+// body and from kMoveByFour particles on each thread flies four at a time,
+// their loads in flight together (4.2M particles: 38 -> 34 us; 800,000 7.3 ->
+// 7.7, and a call on 20,000 with diffuse faces 16 -> 19 us: the boundaries of a
+// thread's particles come one after the other).
+constexpr uint32_t kMoveByFour = 1500000;
+template <bool BODY, int U>
 __global__ void __launch_bounds__(256) k_move(const __grid_constant__ StepParams p, uint32_t n, uint32_t step) {
-  constexpr int U = BODY ? 1 : 4;
   for (uint32_t base = blockIdx.x * blockDim.x * U; base < n; base += gridDim.x * blockDim.x * U) {
     float3 pos[U], vel[U];
 #pragma unroll
@@ -1028,8 +1030,9 @@ cudaError_t launch_scatter(bool with_state, const SoA& src, SoA dst, const uint3
 
 cudaError_t launch_move(const StepParams& p, uint32_t n, uint32_t step, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
-  if (p.has_geom) k_move<true><<<grid_for(n, 256, 8), 256, 0, stream>>>(p, n, step);
-  else k_move<false><<<grid_for(n, 1024, 8), 256, 0, stream>>>(p, n, step);
+  if (p.has_geom) k_move<true, 1><<<grid_for(n, 256, 8), 256, 0, stream>>>(p, n, step);
+  else if (n < kMoveByFour) k_move<false, 1><<<grid_for(n, 256, 8), 256, 0, stream>>>(p, n, step);
+  else k_move<false, 4><<<grid_for(n, 1024, 8), 256, 0, stream>>>(p, n, step);
   return cudaGetLastError();
 }
 
