@@ -139,9 +139,12 @@ void drop_graph(dsmc_handle* h) {
 // that makes enough tiles for the warps of one wave, fewer on small grids,
 // where a warp's chain of chunks is the kernel's length (order kernel, 16^3
 // cells of 24: 36 us with 32, 13 with 4; 13,824 cells of 8: 16 with 32, 10
-// with 8; 65,536 cells: 18 with 32, 20 with 16), and 16 where they fill a
-// chunk and there are tiles enough to even out (524,288 cells of 6-8: 89 with
-// 32, 84 with 16; 182,250 cells of 9: 37 with 32, 40 with 16).
+// with 8; 65,536 cells: 18 with 32, 20 with 16).  On grids of 379,000 to 758,000
+// cells 16, where they fill a chunk (7.2 per cell of 128 particles): a capsule
+// flow of 524,288 cells at 7.5 and 8.4 particles per cell 73.0 and 81.9 us with
+// 32, 70.3 and 78.1 with 16, a box of 8 89.8 and 88.3; at 6 and 7 per cell 67.5
+// and 77.8 with 32, 68.3 and 77.8 with 16; 294,912 cells of 7 59.0 and 58.7;
+// 1,048,576 cells of 7 and 8 151.8 and 170.1 with 32, 158.9 and 175.5 with 16.
 void apply_variant(dsmc_handle* h, int v) {
   h->variant = v;
   const uint64_t cap = (uint64_t)dsmcb::cell_kernel_chunk_capacity(v);
@@ -151,7 +154,9 @@ void apply_variant(dsmc_handle* h, int v) {
     const uint64_t wave = (uint64_t)dsmcb::num_sms() * 20u;  // resident warps of the default shape
     ct = dsmcb::cell_kernel_w_tile();
     while (ct > 4 && 2u * ((uint64_t)h->cells / ct) < wave) ct >>= 1;
-    if (ct == 32 && (uint64_t)h->cells >= 16u * 8u * wave && 16u * (uint64_t)h->ppc * 10u >= 9u * cap) ct = 16;
+    const double ppc = h->cfg.part_per_cell ? (double)h->cfg.part_per_cell
+                                            : (double)h->cfg.density * h->cell_volume / h->cfg.fnum;
+    if (ct == 32 && h->cells >= 128u * wave && h->cells < 256u * wave && 16.0 * ppc >= 0.9 * (double)cap) ct = 16;
   }
   h->cells_per_tile = ct;
   h->n_tiles = (h->cells + ct - 1) / ct;
