@@ -854,7 +854,7 @@ int dsmc_decode_mse(int m, int n, int k, const void* a, const void* b, const flo
 int dsmc_mlp_forward(const dsmc_mlp* n, const float* x, int batch, void* xb, float* const* z, void* const* h, void* cb,
                      float* y, void* stream) {
   if (!n || !x || batch <= 0 || !xb || !h || !cb || n->depth < 0 || n->n_in <= 0 ||
-      n->in_pad < n->n_in || n->n_in > 4096)
+      n->in_pad < n->n_in || n->n_in > 4096 || (n->depth == 0 && n->hidden != n->in_pad))
     return DSMC_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   // as many rows per launch as the parameters hold

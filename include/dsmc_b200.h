@@ -551,9 +551,9 @@ int dsmc_decode_mse(int m, int n, int k, const void* a, const void* b, const flo
                     unsigned long long* count, void* stream);
 /* The network's forward pass in one call: `batch` rows of n_in inputs in host
  * memory (taken before the call returns), padded to in_pad columns; depth
- * layers of `hidden` GELU units; `modes` coefficients; the field, unless y is
- * NULL.  Weights in BF16 (in_pad or hidden x hidden, hidden x modes, modes x
- * fields), biases in FP32.  xb receives the padded inputs, h[l] the
+ * layers of `hidden` GELU units (with none, hidden equals in_pad); `modes`
+ * coefficients; the field, unless y is NULL.  Weights in BF16 (in_pad or
+ * hidden x hidden, hidden x modes, modes x fields), biases in FP32.  xb receives the padded inputs, h[l] the
  * activations and cb the coefficients in BF16, z[l] (z may be NULL) the
  * pre-activations in FP32; device pointers, rows without padding. */
 typedef struct dsmc_mlp {
