@@ -139,8 +139,9 @@ __device__ __forceinline__ void issue_wchunk(const StepParams& p, Smem& S, const
 }
 
 // A cell too large for a chunk: the warp gathers it in sorted order into the
-// mid arrays in global memory; its pairs are collided by one lane of k_ntc_w
-// (the cell is listed as a light cell whatever its pair count).
+// mid arrays in global memory.  In the Philox mode a warp of k_ntc_w collides
+// its pairs (ntc_select_fast_warp: the same selections as one lane's), below
+// kHeavyMin of them and in the reference's streams one lane does.
 static __device__ __noinline__ void giant_order_warp(const StepParams& p, uint32_t s, uint32_t e) {
   const uint32_t n = e - s;
   const uint32_t lane = lane_id();
@@ -533,8 +534,7 @@ constexpr uint32_t kNtcClaim = 256;  // claim slots per warp: the largest chunk
 // 20 -> 14 us; 65,536 cells: 24 -> 18 us; the claims of 3,500 warps on one
 // counter were the difference).  A dense cell's velocities sit in shared
 // memory and its random words come a block at a time (64x32x32 sphere flow,
-// 27 -> 19 us with the claims).  The two-CTA register cap keeps it free of
-// spills: 3 CTAs ran the sphere flow's 3 us slower, the capsule's 1 us faster.
+// 27 -> 19 us with the claims).  RNG and STAGED: launch_ntc_w.
 template <int WARPS, int RNG, bool STAGED>
 __device__ __forceinline__ void ntc_body(const StepParams& p, const uint32_t vb, const uint32_t vg) {
   constexpr bool kDense = RNG != 0;  // the reference's streams have no dense cells
@@ -1320,7 +1320,7 @@ cudaError_t launch_flight_pw(const StepParams& p, cudaStream_t stream) {
 }
 
 constexpr int kNtcWarps = 8;
-constexpr int kNtcWarpsB = 4;  // batched: 20 warps per SM without spills
+constexpr int kNtcWarpsB = 4;  // batched: 20 warps per SM, 20 bytes spilled
 
 template <int WARPS, int RNG, int MINB, bool STAGED>
 cudaError_t launch_ntc_shape(const StepParams& p, cudaStream_t stream) {

@@ -22,8 +22,14 @@ namespace dsmcb {
 
 // Launches `kernel` with programmatic stream serialization: its CTAs may be
 // dispatched while the previous kernel in the stream drains; the kernel must
-// call chained_entry() before touching memory.  Kernel nodes captured into
-// a graph keep the programmatic edge.  The batched (ensemble) stages launch
+// call chained_entry() before touching memory.  Exceptions, each touching only
+// data that the kernel before it does not write (and writing none that it
+// reads): the GEMM's first loads of its weights, kernels launched beside the
+// one before them (beside_entry, which then end after it), and the sampling
+// kernel at the end of a step graph.  They rest on what came before that
+// kernel being complete, which holds as it lets its dependents start only
+// after its own wait, or was launched beside one that did, or unchained.
+// Kernel nodes captured into a graph keep the programmatic edge.  The batched (ensemble) stages launch
 // with chained = false: there the early CTAs of the next stage cost more than
 // they save (1.78 against 2.10 ms per step of the 64-member ensemble), while
 // a single instance gains about 1 %.

@@ -57,18 +57,6 @@ __device__ __forceinline__ void warp_count_key_global(uint32_t* count, uint32_t 
   if ((int)lane == __ffs(tpeers) - 1) atomicAdd(&tile_sum[tk], (uint32_t)__popc(tpeers));
 }
 
-// Ticket from a per-key counter, aggregated over the lanes of `mask` holding
-// the same key.
-__device__ __forceinline__ uint32_t warp_ticket(uint32_t* counter, uint32_t key, unsigned mask) {
-  const unsigned peers = __match_any_sync(mask, key);
-  const int leader = __ffs(peers) - 1;
-  const unsigned lane = lane_id();
-  uint32_t base = 0;
-  if ((int)lane == leader) base = atomicAdd(&counter[key], (uint32_t)__popc(peers));
-  base = __shfl_sync(mask, base, leader);
-  return base + __popc(peers & ((1u << lane) - 1u));
-}
-
 __device__ __forceinline__ void flush_tile_hist(uint32_t* s_tile, uint32_t* tile_sum, uint32_t n) {
   for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
     const uint32_t v = s_tile[t];
