@@ -249,7 +249,10 @@ struct TargetWalk {
   }
 };
 
-template <int BN, bool MSE>
+// PLAIN: some output does not go out by TMA (a form of its own: with that code
+// in it the kernel takes 14 to 40 registers more, and a prediction of one
+// condition 80 us instead of 73).
+template <int BN, bool MSE, bool PLAIN>
 __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
     k_gemm(const __grid_constant__ GemmArgs g, const __grid_constant__ CUtensorMap map_a,
            const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
@@ -467,7 +470,7 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
           for (int i = 0; i < 8; i++)
             *reinterpret_cast<float4*>(fst + 4096 * buf + chunk128(lane, i)) =
                 make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          if (!MSE && !g.tma_c) {
+          if (PLAIN && !g.tma_c) {
             __syncwarp();
             rows_out(g, fst + 4096 * buf, row0, c0);
             __syncwarp();
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(Shape<BN, MSE>::kThreads, 1)
               *reinterpret_cast<uint4*>(hst + 2048 * buf + chunk64(lane, i)) =
                   make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
           }
-          if (!MSE && !g.tma_cb) {
+          if (PLAIN && !g.tma_cb) {
             __syncwarp();
             rows_out_bf16(g, hst + 2048 * buf, row0, c0);
             __syncwarp();
@@ -693,7 +696,7 @@ bool make_map(CUtensorMap* map, bool f32, const void* base, int rows, int cols, 
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool MSE>
+template <int BN, bool MSE, bool PLAIN>
 cudaError_t launch_shape(const GemmArgs& g, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c,
                          const CUtensorMap& cb, const CUtensorMap& t, uint32_t items, cudaStream_t s) {
   static bool set[64] = {};
@@ -703,11 +706,11 @@ cudaError_t launch_shape(const GemmArgs& g, const CUtensorMap& a, const CUtensor
   const int smem = (int)sizeof(Smem<BN, MSE>);
   static_assert(sizeof(Smem<BN, MSE>) <= 227 * 1024, "shared memory of one CTA");
   if (!set[dev & 63]) {
-    e = cudaFuncSetAttribute(k_gemm<BN, MSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(k_gemm<BN, MSE, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     set[dev & 63] = true;
   }
-  return launch_chained(k_gemm<BN, MSE>, std::min<uint32_t>(items, (uint32_t)num_sms()), Shape<BN, MSE>::kThreads, smem, s, true, g,
+  return launch_chained(k_gemm<BN, MSE, PLAIN>, std::min<uint32_t>(items, (uint32_t)num_sms()), Shape<BN, MSE>::kThreads, smem, s, true, g,
                         a, b, c, cb, t);
 }
 
@@ -750,15 +753,20 @@ int run(GemmArgs g, const void* a, int lda, int a_trans, const void* b, int ldb,
              make_map(&mcb, false, g.cb, g.m, g.n, g.ldcb, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
   g.tma_t = MSE && aligned16(g.t) && g.ldt % 8 == 0 &&
             make_map(&mt, false, g.t, g.m, g.n, g.ldt, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+  const uint32_t count = (uint32_t)n_items;
   cudaError_t e;
-  if constexpr (!MSE) {
-    if (bn == 256) {
-      e = launch_shape<256, false>(g, ma, mb, mc, mcb, mt, (uint32_t)n_items, s);
-      return e == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
-    }
+  if constexpr (MSE) {  // (its plain stores are in the one form)
+    e = bn == 128 ? launch_shape<128, true, false>(g, ma, mb, mc, mcb, mt, count, s)
+                  : launch_shape<64, true, false>(g, ma, mb, mc, mcb, mt, count, s);
+  } else if ((g.c && !g.tma_c) || (g.cb && !g.tma_cb)) {
+    e = bn == 256   ? launch_shape<256, false, true>(g, ma, mb, mc, mcb, mt, count, s)
+        : bn == 128 ? launch_shape<128, false, true>(g, ma, mb, mc, mcb, mt, count, s)
+                    : launch_shape<64, false, true>(g, ma, mb, mc, mcb, mt, count, s);
+  } else {
+    e = bn == 256   ? launch_shape<256, false, false>(g, ma, mb, mc, mcb, mt, count, s)
+        : bn == 128 ? launch_shape<128, false, false>(g, ma, mb, mc, mcb, mt, count, s)
+                    : launch_shape<64, false, false>(g, ma, mb, mc, mcb, mt, count, s);
   }
-  if (bn == 128) e = launch_shape<128, MSE>(g, ma, mb, mc, mcb, mt, (uint32_t)n_items, s);
-  else e = launch_shape<64, MSE>(g, ma, mb, mc, mcb, mt, (uint32_t)n_items, s);
   return e == cudaSuccess ? DSMC_OK : DSMC_ERR_CUDA;
 }
 
