@@ -398,29 +398,30 @@ __global__ void __launch_bounds__(256) k_scatter_kv(const uint32_t* __restrict__
 // Restores input order within each key: entry of rank r (by input position)
 // among its key's entries goes to start[key] + r.  A CTA takes kt keys at a
 // time (at most kFixupThreads), in chunks of whole keys of at most kFixupCap
-// entries in shared memory; tiles are small (launch_segment_fixup), so that a
+// entries in shared memory; tiles are small (launch_sort), so that a
 // few thousand keys reach every SM (4,096 keys of 24: 35 us with tiles of 256
 // keys on 16 CTAs, now 5 us; 524,288 keys of 8: 58, now 34 us).
-constexpr int kFixupThreads = 128, kFixupCap = 1024;
+constexpr int kFixupThreads = 128, kFixupCap = 768;
 
-// Keys with more than kLargeKey entries are ranked by themselves: entries
-// [i0, i0 + Q kFixupThreads) of such a key, m at s0 (the whole CTA).  Each
-// thread ranks Q of them against the key's positions, kFixupCap at a time in
-// shared memory, four per load.  Bound by the comparisons, m squared of them:
-// 4.2M entries of which 1 % are in keys of 2,500, 524,288 keys: 4.2 ms with
-// chunks of 4,096 entries and 256 threads, 4.4 with chunks of 1,024 and larger
-// keys ranked from global memory, now 1.9; 256 keys of 16,384 4.7 s -> 53 ms.
-constexpr uint32_t kLargeKey = 256;
-template <int Q, bool PAIR>
+// A key with more than kFixupCap entries (m at s0, the whole CTA): its entries
+// [i0, i1), at most 4 kFixupThreads, are ranked against the key's positions,
+// kFixupCap at a time in shared memory.  Each thread ranks up to four entries
+// and reads four positions per load: bound by the comparisons, m squared of
+// them (1,000,000 entries in 400 keys 57 ms with chunks of 4,096 and 256
+// threads, 3.3 ms with chunks of 1,024 and such keys ranked from global memory,
+// now 0.53; 4.2M entries in 524,288 keys, 1 % of them in keys of 2,500, 4.1, 4.4
+// and 2.5 ms).  Eight entries per thread take 1.9 ms for the latter, but
+// registers that cost every sort 4 %; a kernel of its own costs its launch.
+template <bool PAIR>
 __device__ __forceinline__ void rank_large_key(uint32_t* spos, const ScatterOut<PAIR>& in, uint32_t s0, uint32_t m,
-                                               uint32_t i0, uint32_t key, uint32_t* keys_out, uint32_t* vals_out) {
-  uint32_t my[Q], val[Q], rank[Q];
+                                               uint32_t i0, uint32_t i1, uint32_t key, uint32_t* keys_out,
+                                               uint32_t* vals_out) {
+  constexpr int Q = 4;
+  uint32_t my[Q], rank[Q];
 #pragma unroll
   for (int q = 0; q < Q; q++) {
     const uint32_t t = i0 + threadIdx.x + q * kFixupThreads;
-    const uint2 e = t < m ? in.get(s0 + t) : make_uint2(0u, 0u);
-    val[q] = e.x;
-    my[q] = e.y;
+    my[q] = t < i1 ? in.position(s0 + t) : 0u;
     rank[q] = 0;
   }
   for (uint32_t j0 = 0; j0 < m; j0 += kFixupCap) {
@@ -439,9 +440,10 @@ __device__ __forceinline__ void rank_large_key(uint32_t* spos, const ScatterOut<
   }
 #pragma unroll
   for (int q = 0; q < Q; q++) {
-    if (i0 + threadIdx.x + q * kFixupThreads >= m) break;
+    const uint32_t t = i0 + threadIdx.x + q * kFixupThreads;
+    if (t >= i1) break;
     keys_out[s0 + rank[q]] = key;
-    vals_out[s0 + rank[q]] = val[q];
+    vals_out[s0 + rank[q]] = in.get(s0 + t).x;
   }
 }
 
@@ -453,7 +455,6 @@ __global__ void __launch_bounds__(kFixupThreads) k_segment_fixup(const uint32_t*
   __shared__ uint32_t ls[kFixupThreads + 1];
   __shared__ __align__(16) uint32_t spos[kFixupCap];
   __shared__ uint8_t cellof[kFixupCap];  // the chunk's key of each entry
-  __shared__ uint32_t first;
   const uint32_t ntiles = (nkeys + kt - 1) / kt;
   for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint32_t c0 = tile * kt, nct = min(kt, nkeys - c0);
@@ -465,29 +466,12 @@ __global__ void __launch_bounds__(kFixupThreads) k_segment_fixup(const uint32_t*
       const uint32_t base = ls[cur];
       const uint32_t c = cur + 1 + threadIdx.x;
       const int fits = (c <= nct) && (ls[c] - base <= (uint32_t)kFixupCap);
-      uint32_t k = __syncthreads_count(fits);
-      // a chunk ends before a large key
-      const bool large = threadIdx.x <= k && c <= nct && ls[c] - ls[c - 1] > kLargeKey;
-      if (__syncthreads_or(large)) {
-        if (threadIdx.x == 0) first = k;
-        __syncthreads();
-        if (large) atomicMin(&first, threadIdx.x);
-        __syncthreads();
-        k = first;
-      }
-      if (k == 0) {
-        // one large key, in passes of nearly equal size
-        const uint32_t m = ls[cur + 1] - base, key = c0 + cur;
-        const uint32_t passes = (m + kFixupCap - 1) / kFixupCap;
-        const uint32_t q = (m + passes * kFixupThreads - 1) / (passes * kFixupThreads);  // entries per thread
-        for (uint32_t i0 = 0; i0 < m; i0 += q * kFixupThreads) {
-          if (q <= 3) rank_large_key<3>(spos, in, base, m, i0, key, keys_out, vals_out);
-          else if (q == 4) rank_large_key<4>(spos, in, base, m, i0, key, keys_out, vals_out);
-          else if (q == 5) rank_large_key<5>(spos, in, base, m, i0, key, keys_out, vals_out);
-          else if (q == 6) rank_large_key<6>(spos, in, base, m, i0, key, keys_out, vals_out);
-          else if (q == 7) rank_large_key<7>(spos, in, base, m, i0, key, keys_out, vals_out);
-          else rank_large_key<8>(spos, in, base, m, i0, key, keys_out, vals_out);
-        }
+      const uint32_t k = __syncthreads_count(fits);
+      if (k == 0) {  // a key above the chunk, in passes of nearly equal size
+        const uint32_t m = ls[cur + 1] - base, passes = (m + 4 * kFixupThreads - 1) / (4 * kFixupThreads);
+        const uint32_t per = (m + passes * kFixupThreads - 1) / (passes * kFixupThreads) * kFixupThreads;
+        for (uint32_t i0 = 0; i0 < m; i0 += per)
+          rank_large_key(spos, in, base, m, i0, min(m, i0 + per), c0 + cur, keys_out, vals_out);
         cur += 1;
         __syncthreads();
         continue;
@@ -1057,6 +1041,9 @@ cudaError_t launch_sort(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t nke
   // 8 on small key ranges
   uint32_t kt = 64;
   while (kt > 8 && nkeys / kt < (uint32_t)num_sms() * 8u) kt >>= 1;
+  // nor more than a chunk of entries on the average (10,000 entries in 8 keys: 846
+  // us on one CTA, 77 on eight)
+  while (kt > 1 && (uint64_t)n * kt > (uint64_t)nkeys * kFixupCap) kt >>= 1;
   const uint32_t ft = (nkeys + kt - 1) / kt, fgrid = std::min(ft, (uint32_t)num_sms() * 16u);
   const uint32_t sgrid = grid_for(n, 1024, 8);
   if (((uintptr_t)scratch & 7u) == 0) {

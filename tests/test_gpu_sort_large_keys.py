@@ -1,6 +1,6 @@
-"""Stable sort with keys that the fixup ranks by themselves (more than 256
-entries) and of more entries than its chunk (1,024), at the edges of its
-passes, beside small and empty keys."""
+"""Stable sort with keys of up to and above the fixup's chunk (768 entries),
+which are ranked by themselves, at the edges of their passes (512 entries),
+beside small and empty keys."""
 import numpy as np
 import pytest
 import torch
@@ -10,7 +10,7 @@ from cudadsmc_b200 import stages
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("large", [[255, 256, 256], [257, 384, 385], [300] * 40, [512, 513, 641], [897, 1024], [1025], [1280, 1281], [1535, 1536, 1537], [1793], [2047, 2048, 2049, 3],
+@pytest.mark.parametrize("large", [[255, 256, 256], [257, 384, 385], [300] * 40, [512, 513, 641], [767, 768, 769], [897, 1024], [1025], [1280, 1281], [1535, 1536, 1537], [1793], [2047, 2048, 2049, 3],
                                    [4096, 4097], [30000, 1100]])
 @pytest.mark.parametrize("form", ["aligned", "off4", "static"])
 def test_large_keys(cuda, large, form):
