@@ -1322,8 +1322,9 @@ cudaError_t launch_flight_pw(const StepParams& p, cudaStream_t stream) {
 constexpr int kNtcWarps = 8;
 constexpr int kNtcWarpsB = 4;  // batched: 20 warps per SM, 20 bytes spilled
 
+// smem: shared memory asked for beyond the kernel's own.
 template <int WARPS, int RNG, int MINB, bool STAGED>
-cudaError_t launch_ntc_shape(const StepParams& p, cudaStream_t stream) {
+cudaError_t launch_ntc_shape(const StepParams& p, cudaStream_t stream, size_t smem = 0) {
   static LaunchShapeW cache[8];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1331,20 +1332,30 @@ cudaError_t launch_ntc_shape(const StepParams& p, cudaStream_t stream) {
   LaunchShapeW& ls = cache[dev & 7];
   if (ls.device != dev) {
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ntc_w<WARPS, RNG, MINB, STAGED>, WARPS * 32, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ntc_w<WARPS, RNG, MINB, STAGED>, WARPS * 32, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     ls.device = dev;
     ls.per_sm = per_sm;
   }
-  return launch_chained(k_ntc_w<WARPS, RNG, MINB, STAGED>, (uint32_t)(num_sms() * ls.per_sm), WARPS * 32, 0, stream,
-                        Chain(true, p.carveout), p);
+  return launch_chained(k_ntc_w<WARPS, RNG, MINB, STAGED>, (uint32_t)(num_sms() * ls.per_sm), WARPS * 32, smem,
+                        stream, Chain(true, p.carveout), p);
 }
 cudaError_t launch_ntc_w(const StepParams& p, cudaStream_t stream) {
-  // Reference streams: light cells only, so 72 registers and 3 CTAs (a form
-  // for both kinds of stream takes 104 and 2).  12.8M particles, 1.6M cells:
-  // step 774 -> 735 us; 524,288 of 8 249 -> 237; 16^3 cells of 24 48.5 -> 44.1.
-  if (p.rng_kind == 0) return launch_ntc_shape<kNtcWarps, 0, 3, false>(p, stream);
+  const uint32_t lanes = (uint32_t)num_sms() * 16u * 32u;  // of 16 warps per SM
+  if (p.rng_kind == 0) {
+    // Reference streams: light cells only, so 72 registers and 24 warps per SM
+    // (the form for both kinds of stream takes 104 and 16 warps): 12.8M
+    // particles in 1.6M cells, step 774 -> 735 us; 524,288 cells of 8 249 -> 237;
+    // 16^3 cells of 24 48.5 -> 44.  Not where the cells are two rounds of lanes
+    // either way (147,456 of 30: 315 against 335).  The 16 KB keep the split of
+    // L1 and shared memory that the kernels before and after it have: next to
+    // nothing asked for, the SMs are set up anew in between (64,000 cells of 30
+    // 157 -> 176 us, 8^3 cells of 260 301 -> 387).
+    const bool two = p.cells > lanes / 2u * 3u && p.cells <= 2u * lanes;
+    return two ? launch_ntc_shape<kNtcWarps, -1, 2, true>(p, stream)
+               : launch_ntc_shape<kNtcWarps, 0, 3, false>(p, stream, 16384);
+  }
   // Philox: 16 warps per SM, or 20 in smaller CTAs where the light cells are
   // many times the lanes (1.6M cells of 8: 108 -> 100 us, 524,288 of 8 42.2 ->
   // 39.9, 196,608 of 8 21.9 -> 21.3), but not for fewer cells (147,456 of 8: 18.6
@@ -1353,9 +1364,8 @@ cudaError_t launch_ntc_w(const StepParams& p, cudaStream_t stream) {
   // how many are under way, not each one's chain: 24 warps, velocities in
   // place (524,288 cells of 30: 388 -> 316 us, of 24 151 -> 137; 110,592 of 20 32.7
   // -> 39.4, a sphere flow of 524,288 of 21 59.5 -> 64.5).
-  const float lanes = (float)num_sms() * 16.f * 32.f, cells = (float)p.cells;
-  if (cells >= 5.f * lanes && p.avg_conc >= 24.f) return launch_ntc_shape<kNtcWarps, 1, 3, false>(p, stream);
-  if (cells >= 2.5f * lanes && p.avg_conc < 14.f) return launch_ntc_shape<4, 1, 5, true>(p, stream);
+  if (p.cells >= 5u * lanes && p.avg_conc >= 24.f) return launch_ntc_shape<kNtcWarps, 1, 3, false>(p, stream);
+  if (p.cells >= lanes / 2u * 5u && p.avg_conc < 14.f) return launch_ntc_shape<4, 1, 5, true>(p, stream);
   return launch_ntc_shape<kNtcWarps, 1, 2, true>(p, stream);
 }
 

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 # 148 SMs of 16 warps: lines at 189,440 and 378,880 cells, 14 and 24 per cell
 CASES = [((57, 57, 57), 5, "philox"), ((58, 58, 58), 5, "philox"), ((58, 58, 58), 14, "philox"),
          ((72, 72, 72), 24, "philox"), ((73, 73, 73), 24, "philox"), ((20, 20, 20), 24, "philox"),
-         ((58, 58, 58), 5, "taus"), ((20, 20, 20), 30, "taus"), ((3, 2, 2), 90, "taus")]
+         ((58, 58, 58), 5, "taus"), ((20, 20, 20), 30, "taus"), ((3, 2, 2), 90, "taus"),
+         # reference streams: another form from 113,665 to 151,552 cells
+         ((48, 48, 49), 9, "taus"), ((48, 48, 50), 9, "taus"), ((53, 53, 54), 9, "taus")]
 
 
 @pytest.mark.parametrize("dim,ppc,rng", CASES)
